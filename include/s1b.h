@@ -443,7 +443,8 @@ int s1b_los_grid(const s1b_orbit_poly_t *orbit, double t0, double lat0, double l
 /* ------------------------------------------------------------ burst stitching */
 
 /* One burst interferogram of a frame: `offset` = first element in the data
- * buffer (bursts back to back, row-major [bottom - top x right - left]);
+ * buffer (row-major [bottom - top x right - left]; the bursts may lie
+ * anywhere from `data` on, back to back or not);
  * left/top/right/bottom in frame pixels; subswath 1..3; `group` identifies
  * the pair of burst ids (the overlap phase offset is estimated when it
  * changes from the previous burst, s1proc/interfere.py:92-118). */
@@ -453,7 +454,7 @@ typedef struct {
   int32_t subswath, group;
 } s1b_stitch_burst_t;
 
-/* Device workspace of s1b_stitch (subswath mosaics and tables). */
+/* Device workspace of s1b_stitch (offsets, measured overlaps, tables). */
 size_t s1b_stitch_workspace_bytes(const s1b_stitch_burst_t *bursts, int32_t n, int32_t out_float);
 
 /* Stitch burst interferograms (complex64, or float32 phase with out_float)
@@ -464,7 +465,8 @@ size_t s1b_stitch_workspace_bytes(const s1b_stitch_burst_t *bursts, int32_t n, i
  * non-zero.  bursts: host array; offsets_host (optional, double [n]): the
  * offset applied to each burst (synchronises the stream when given).  The
  * union box of a subswath is that of its first and last burst, as the
- * reference computes it; parts of middle bursts outside it are dropped. */
+ * reference computes it; parts of middle bursts outside it are dropped.
+ * `frame` must not overlap the bursts. */
 int s1b_stitch(const s1b_stitch_burst_t *bursts, int32_t n, const void *data, int32_t out_float, int32_t nrow0,
                int32_t ncol0, void *frame, double *offsets_host, void *workspace, size_t workspace_bytes,
                void *stream);

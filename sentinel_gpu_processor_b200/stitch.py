@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 import numpy as np
 import torch
@@ -27,24 +28,33 @@ def stitch_bursts(bursts, nrow0, ncol0, out_float=False, return_offsets=False):
     if not bursts:
         raise ValueError("no bursts")
     dev = bursts[0][1].device
-    parts, table, off = [], [], 0
+    # the kernels read every burst where it lies: its offset is the distance of
+    # its tensor from the first one in memory, in elements (no gathered copy)
+    es, n = dtype.itemsize, len(bursts)
+    parts, flat = [], []
     for (l, t, r, b), d, sw, grp in bursts:
-        d = d.to(dtype).contiguous()
-        if tuple(d.shape) != (b - t, r - l):
+        if d.device != dev or not d.is_cuda:
+            raise ValueError("bursts must be CUDA tensors of one device")
+        if d.shape != (b - t, r - l):
             raise ValueError("burst data does not match its box")
-        parts.append(d.reshape(-1))
-        table.append(_lib.StitchBurst(off, int(l), int(t), int(r), int(b), int(sw), int(grp)))
-        off += d.numel()
-    data = torch.cat(parts)
-    arr = (_lib.StitchBurst * len(table))(*table)
+        if d.dtype != dtype or not d.is_contiguous() or d.is_conj() or d.is_neg():
+            d = d.to(dtype).contiguous().resolve_conj().resolve_neg()
+        parts.append(d)
+        flat += (d.data_ptr(), int(l), int(t), int(r), int(b), int(sw), int(grp))
+    base = min(flat[::7])
+    for i in range(0, 7 * n, 7):
+        flat[i], odd = divmod(flat[i] - base, es)
+        if odd:
+            raise ValueError("burst data must be aligned to its elements")
+    arr = (_lib.StitchBurst * n).from_buffer_copy(struct.pack("=" + "q6i" * n, *flat))
     lib = _lib.load()
-    ws_bytes = int(lib.s1b_stitch_workspace_bytes(arr, len(table), 1 if out_float else 0))
+    ws_bytes = int(lib.s1b_stitch_workspace_bytes(arr, n, 1 if out_float else 0))
     if ws_bytes == 0:
         raise ValueError("bad burst table")
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     frame = torch.empty((nrow0, ncol0), dtype=dtype, device=dev)
-    offs = (ctypes.c_double * len(table))() if return_offsets else None
-    _lib.check(lib.s1b_stitch(arr, len(table), _lib.dptr(data), 1 if out_float else 0, int(nrow0), int(ncol0),
+    offs = (ctypes.c_double * n)() if return_offsets else None
+    _lib.check(lib.s1b_stitch(arr, n, ctypes.c_void_p(base), 1 if out_float else 0, int(nrow0), int(ncol0),
                               _lib.dptr(frame), offs, _lib.dptr(ws), ws_bytes, _lib.stream_ptr()), "s1b_stitch")
     if return_offsets:
         return frame, list(offs)
