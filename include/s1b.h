@@ -235,6 +235,18 @@ int s1b_deramp_ci16(const s1b_burst_plan_t *plan, const void *in, void *out, voi
 int s1b_geo2rdr(const s1b_burst_plan_t *plan, const int16_t *dem, int64_t dem_pitch,
                 const void *deramped, void *out, int32_t *rows, void *stream);
 
+/* s1b_deramp and s1b_geo2rdr in one: a burst's raw samples geocoded onto the
+ * plan's DEM window, deramped where they are gathered (no deramped copy; the
+ * same values within float32 rounding).
+ *   slc:     [lines * samples] device, complex64 (S1B_SAMPLES_C64) or complex
+ *            int16 (S1B_SAMPLES_CI16).
+ *   dem, dem_pitch, out, rows: as in s1b_geo2rdr.
+ *   scratch: device, s1b_geocode_scratch_bytes(plan) bytes, 16-byte aligned
+ *            (24 bytes per burst column). */
+size_t s1b_geocode_scratch_bytes(const s1b_burst_plan_t *plan);
+int s1b_geocode(const s1b_burst_plan_t *plan, const void *slc, int32_t sample_format, const int16_t *dem,
+                int64_t dem_pitch, void *out, int32_t *rows, void *scratch, size_t scratch_bytes, void *stream);
+
 /* Sample coordinates of every pixel of the plan's DEM window as the
  * geocoding solves them (per-warp orbit patch, line-model seeds, chord
  * Newton, in the frame's 128-row tiles, every pixel solved): az = line,

@@ -144,6 +144,9 @@ _SIGNATURES = {
     "s1b_deramp": (c_int, [POINTER(BurstPlan), c_void_p, c_void_p, c_void_p]),
     "s1b_deramp_ci16": (c_int, [POINTER(BurstPlan), c_void_p, c_void_p, c_void_p]),
     "s1b_geo2rdr": (c_int, [POINTER(BurstPlan), c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "s1b_geocode_scratch_bytes": (c_size_t, [POINTER(BurstPlan)]),
+    "s1b_geocode": (c_int, [POINTER(BurstPlan), c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
+                            c_size_t, c_void_p]),
     "s1b_set_geocode_culling": (c_int, [c_int32]),
     "s1b_zero_doppler": (c_int, [POINTER(OrbitPoly), c_void_p, c_int64, c_double, c_void_p, c_void_p, c_void_p]),
     "s1b_llh2xyz": (c_int, [c_void_p, c_void_p, c_int64, c_void_p]),

@@ -12,6 +12,7 @@
 //   * llh->ECEF trigonometry is computed once per DEM row / column per warp;
 //   * FP64 phases are reduced mod 2 pi in FP64, then rotated in FP32;
 //   * the non-zero-row search is folded into the geocoding epilogue.
+#include <algorithm>
 #include <climits>
 #include <cstddef>
 #include <type_traits>
@@ -226,6 +227,11 @@ __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float f) {
   return make_float2(fmaf(f, b.x - a.x, a.x), fmaf(f, b.y - a.y, a.y));
 }
 
+// lerp2 with paired FP32 operations (the same values).
+__device__ __forceinline__ float2 lerp2p(float2 a, float2 b, float f) {
+  return __ffma2_rn(make_float2(f, f), __ffma2_rn(make_float2(-1.f, -1.f), a, b), a);
+}
+
 // Read-only (L1-cached) sample loads for the bilinear gathers.
 __device__ __forceinline__ float2 load_ro(const float2 *p) { return __ldg(p); }
 __device__ __forceinline__ float2 load_ro(const short2 *p) {
@@ -266,7 +272,7 @@ struct GeoConsts {
 };
 
 template <typename PL>
-__device__ __forceinline__ GeoConsts geo_consts(const PL &P) {
+__host__ __device__ __forceinline__ GeoConsts geo_consts(const PL &P) {
   return GeoConsts{1.0 / P.dmrg, 1.0 / P.dtaz, 2.0 / kSolD, 4.0 / P.wvl,
                    (double)P.first_valid_sample, (double)(P.last_valid_sample - 1),
                    (double)(P.first_valid_line + 5), (double)(P.last_valid_line - 5),
@@ -391,7 +397,7 @@ __device__ __forceinline__ unsigned geo_warp_setup(const PL &P, const s1b_orbit_
   if (__all_sync(0xffffffffu, conv) && cull && resid < 1.0 && slack < 1.0e4) {
     const double zcs = zc * (cR - cL);  // the model's change across the warp's columns
 #pragma unroll
-    for (int j = 0; j < RY / 32; ++j) {
+    for (int j = 0; j < (RY + 31) / 32; ++j) {
       const int ra = max(32 * j, rTr), re = min(32 * j + 32, rBr + 1);
       const double za = zTL + zr * (ra - rTr), zb = zTL + zr * (re - 1 - rTr);
       const double lo = fmin(za, zb) + fmin(zcs, 0.0) - slack, hi = fmax(za, zb) + fmax(zcs, 0.0) + slack;
@@ -570,6 +576,205 @@ __global__ __launch_bounds__(G_TX) void geo2rdr_kernel(
     const float2 *__restrict__ burst, float2 *__restrict__ out, int32_t *__restrict__ rows,
     int nrow, int ncol, bool cull) {
   geo2rdr_tile<G_TX, G_RY>(P, P.orbit, dem, pitch, burst, out, rows, nrow, ncol, blockIdx.x, blockIdx.y, cull);
+}
+
+// ------------------------------------------------- geocoding, one launch
+// Deramp and geocoding of one burst without the deramped copy: the raw
+// samples (complex64 or complex int16) are deramped where they are gathered,
+// as in the frame's geocoding, but with FP64 phases throughout (phases within
+// ~1e-8 rad before their FP32 rotation).
+//
+// Per pixel and burst:
+//   * ECEF point from row terms (in shared memory, once per CTA) and column
+//     terms: rho = (re + h) cos lat, z = (re (1 - e^2) + h) sin lat;
+//   * the patch's dot products in cylindrical form: with the thread's column
+//     fixed, d.v = rho (v0 cos lon + v1 sin lon) + z v2 - x.v is two
+//     multiply-adds instead of three and the subtractions of d (the products
+//     reach 5e10 and round to 4e-6, 6e-14 s of time; the squared range, which
+//     the phase needs to 1e-15, keeps the differences d);
+//   * two chord steps from the line model's seed, the stopping test after;
+//   * the deramp of a gathered line and the pixel's reramp as one phase formed
+//     from small differences: with u = eta_line - etaref_c0, w the pixel's
+//     eta - etaref less u, K = kt,
+//       kt_p (u + w)^2 - K0 u^2 = K0 w (2u + w) + frd (K1 - K0) (u + w)^2.
+// What bounds it is instruction issue (68 % of slots, FP64 pipe 36 %): 1500 x
+// 21000 complex int16 samples onto 16 M window pixels in 185 us, against 85 us
+// for the deramp and 230 us for the geocoding of the deramped copy; 64-row
+// tiles 193 us, 6 CTAs of two rows per trip 205 us, no prefetch of the
+// footprint 196 us.
+struct GeoRow {
+  double rho0, coslat, z0, sinlat;  // (rho, z) = (rho0 + h coslat, z0 + h sinlat)
+};
+
+// Per-burst launch constants, formed once on the host.
+struct GeocodeArgs {
+  const int16_t *dem;
+  int64_t pitch;
+  const void *slc;
+  const double2 *tops;   // (-kt, etaref) per burst column
+  const float2 *slopes;  // (kt' - kt, etaref' - etaref) to the next column
+  float2 *out;
+  int32_t *rows;
+  int32_t nrow, ncol, cull;
+  // first valid integer sample and line, and how many there are
+  int32_t rg_first, az_first;
+  uint32_t rg_span, az_span;
+  GeoConsts gc;
+};
+
+// The column tables of a burst, and its crop rows set to "none".
+__global__ __launch_bounds__(128) void geocode_tables_kernel(const __grid_constant__ s1b_burst_plan_t P,
+                                                             double2 *__restrict__ tops, float2 *__restrict__ slopes,
+                                                             int32_t *__restrict__ rows, int nrow) {
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c == 0 && rows) {
+    rows[0] = nrow;
+    rows[1] = -1;
+  }
+  if (c >= P.samples) return;
+  double kt, eref, kt1, eref1;
+  tops_kt(P, c, kt, eref);
+  tops_kt(P, c + 1, kt1, eref1);
+  tops[c] = make_double2(-kt, eref);
+  slopes[c] = make_float2((float)(kt1 - kt), (float)(eref1 - eref));
+}
+
+template <int RY, typename TSrc>
+__global__ __launch_bounds__(G_TX, 5) void geocode_kernel(const __grid_constant__ s1b_burst_plan_t P,
+                                                          const __grid_constant__ GeocodeArgs a) {
+  __shared__ __align__(16) GeoRow s_row[RY];
+  __shared__ ZeroDopplerPatch s_zd[G_TX / 32];
+  __shared__ double4 s_seed[G_TX / 32];
+  const int tx = threadIdx.x, lane = tx & 31, wid = tx >> 5;
+  const int col = blockIdx.x * G_TX + tx, row0 = blockIdx.y * RY;
+  const int rmax = min(RY, a.nrow - row0);
+  if (tx < RY) {
+    double sl, cl;
+    sincos((P.lat0 + (row0 + tx) * P.dlat) * kPiD / 180, &sl, &cl);
+    const double re = kRaD / sqrt(1. - kRe2D * sl * sl);
+    s_row[tx] = GeoRow{re * cl, cl, re * (1 - kRe2D) * sl, sl};
+  }
+  double sinlon, coslon;
+  sincos((P.lon0 + col * P.dlon) * kPiD / 180, &sinlon, &coslon);
+  const bool colok = col < a.ncol;
+  const TSrc *burst = static_cast<const TSrc *>(a.slc);
+  const int c0 = blockIdx.x * G_TX + wid * 32;
+  const unsigned culled = geo_warp_setup<RY>(P, P.orbit, a.dem, a.pitch, burst, row0, row0, row0 + rmax - 1,
+                                             min(c0, a.ncol - 1), min(c0 + 31, a.ncol - 1), a.cull != 0, s_zd[wid],
+                                             s_seed[wid]);
+  __syncthreads();  // row terms, and lane 0's patch and seed model
+  float2 *dst = a.out + (size_t)row0 * a.ncol + col;
+  if (culled) {  // RY <= 32: one block
+    if (colok)
+      for (int r = 0; r < rmax; ++r, dst += a.ncol) __stcs(dst, make_float2(0.f, 0.f));
+    return;
+  }
+  const ZeroDopplerPatch &zd = s_zd[wid];
+  const double4 m = s_seed[wid];
+  const GeoConsts &gc = a.gc;
+  // cylindrical forms at the thread's longitude, and their constant parts
+  const double vl = fma(zd.v[0], coslon, zd.v[1] * sinlon), al = fma(zd.a[0], coslon, zd.a[1] * sinlon);
+  const double jl = fma(zd.jh[0], coslon, zd.jh[1] * sinlon);
+  double xv = 0.0, xa = zd.vv, xj = zd.k2;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    xv = fma(zd.x[i], zd.v[i], xv);
+    xa = fma(zd.x[i], zd.a[i], xa);
+    xj = fma(zd.x[i], zd.jh[i], xj);
+  }
+  const double hb = fma(m.y, i32_to_f64(col), m.x);  // the seed's column term
+  const int16_t *demc = a.dem + (int64_t)row0 * a.pitch + col;
+  int rlo = INT_MAX, rhi = -1;
+  double rd = 0.0;  // r
+  int hn = colok ? __ldg(demc) : 0;
+#pragma unroll 2
+  for (int r = 0; r < rmax; ++r, dst += a.ncol) {
+    const double hgt = i32_to_f64(hn);
+    demc += a.pitch;
+    if (colok && r + 1 < rmax) hn = __ldg(demc);
+    const GeoRow g = s_row[r];
+    const double rho = fma(hgt, g.coslat, g.rho0), z = fma(hgt, g.sinlat, g.z0);
+    ZeroDopplerPoint q;
+    q.c0 = fma(rho, vl, fma(z, zd.v[2], -xv));
+    q.c1 = fma(rho, al, fma(z, zd.a[2], -xa));
+    q.c2 = fma(rho, jl, fma(z, zd.jh[2], -xj));
+    const double d0 = fma(rho, coslon, -zd.x[0]), d1 = fma(rho, sinlon, -zd.x[1]), d2 = z - zd.x[2];
+    q.dd = fma(d0, d0, fma(d1, d1, d2 * d2));
+    // one Newton step from the seed with the slope there, its reciprocal from
+    // the patch centre's by one Newton step of its own (3e-4 -> 1e-7); a seed
+    // far from its root goes on as the reference does
+    double h = fma(m.w, hgt, fma(m.z, rd, hb));
+    rd += 1.0;
+    const double slope = fma(fma(3.0 * zd.c3, h, 2.0 * q.c2), h, q.c1);
+    const double inv = zd.inv_c1 * fma(-slope, zd.inv_c1, 2.0);
+    const double step = inv * fma(fma(fma(zd.c3, h, q.c2), h, q.c1), h, q.c0);
+    h -= step;
+    double r2;
+    if (fabs(step) < 1.0e-4) {
+      r2 = fma(-h, fma(fma(fma(0.5 * zd.c3, h, (2.0 / 3.0) * q.c2), h, q.c1), h, 2.0 * q.c0), q.dd);
+    } else {
+      r2 = zero_doppler_solve(q, zd.c3, zd.inv_c1, h);
+    }
+    const double rng = sqrt_heron(r2), t = zd.t0 + h;
+    const double rgoff = (rng - P.rngstart) * gc.inv_dmrg, azoff = (t - P.tstart) * gc.prf;
+    int intr, inta;
+    double rgi = floor_int(rgoff, intr), azi = floor_int(azoff, inta);
+    double frd = rgoff - rgi;
+    // validity window fvs < rg < lvs - 1, fvl + 5 <= az < lvl - 5
+    // (geo2rdr.cu:208-209) and the 2 x 2 neighbourhood inside the burst even
+    // if those limits exceed the raster, on the integer parts; the FP64 tests
+    // keep what does not fit an int (or is no number) out
+    const bool valid = colok && (unsigned)(intr - a.rg_first) < a.rg_span && (unsigned)(inta - a.az_first) < a.az_span &&
+                       fabs(rgoff) < 1.0e9 && fabs(azoff) < 1.0e9 && (frd > 0.0 || intr > P.first_valid_sample);
+    float2 res = make_float2(0.f, 0.f);
+    if (valid) {
+      // limits below the raster let (-1, 0) in, which the reference's int()
+      // takes to sample (line) 0
+      if (intr < 0) {
+        intr = 0;
+        frd = rgoff;
+      }
+      if (inta < 0) {
+        inta = 0;
+        azi = 0.0;
+      }
+      const TSrc *src = burst + (size_t)inta * P.samples + intr;
+      const float2 s1 = load_ro(src), s2 = load_ro(src + 1);
+      const float2 s3 = load_ro(src + P.samples), s4 = load_ro(src + P.samples + 1);
+      const double2 k = __ldg(a.tops + intr);
+      const float2 dk = __ldg(a.slopes + intr);
+      const float fr = (float)frd, fa = (float)(azoff - azi);
+      const double ea = fma(azi, P.ati, gc.ea0);            // deramp_eta of the line
+      const double u = ea - k.y;                           // line from its column's reference
+      const double w = fma(-frd, (double)dk.y, gc.eta0 + t - P.tstart - ea);
+      const float e = (float)(u + w), uf = (float)u, k0 = -(float)k.x;
+      // the line below: u + ati, w - ati, whose K0 w (2u + w) is less by
+      // K0 ati (2u + ati)
+      const double ha = fma(-k.x, w * fma(2.0, u, w), fma(gc.k4_wvl, rng, (double)(fr * dk.x * e * e)));
+      const double hb2 = fma(k.x, P.ati * fma(2.0, u, P.ati), ha);
+      const float2 pa = phasor_quarter(ha), pb = phasor_quarter(hb2);
+      // the second column's sample of a line turns by the columns' difference
+      // K0 de (2u - de) - dk (u - de)^2 (a few 1e-3 half-cycles: FP32)
+      const float de = dk.y, ufb = uf + gc.ati_f, ua = uf - de, uc = ufb - de;
+      const float ra = fmaf(k0 * de, 2.f * uf - de, -dk.x * ua * ua);
+      const float rb = fmaf(k0 * de, 2.f * ufb - de, -dk.x * uc * uc);
+      const float2 ca = cmul(lerp2p(s1, cmul(s2, rotation_pi_f(ra)), fr), pa);
+      const float2 cb = cmul(lerp2p(s3, cmul(s4, rotation_pi_f(rb)), fr), pb);
+      res = lerp2p(ca, cb, fa);
+    }
+    if (colok) __stcs(dst, res);
+    if (res.x != 0.f || res.y != 0.f) {
+      rlo = min(rlo, row0 + r);
+      rhi = row0 + r + 1;
+    }
+  }
+  // first / last non-zero output row (geo2rdr.cu:86-128), one reduction pair per warp
+  rlo = __reduce_min_sync(0xffffffffu, rlo);
+  rhi = __reduce_max_sync(0xffffffffu, rhi);
+  if (lane == 0 && a.rows && rhi >= 0) {
+    atomicMin(a.rows, rlo);
+    atomicMax(a.rows + 1, rhi);
+  }
 }
 
 // Zero-Doppler sample coordinates of every DEM pixel of a burst's window, as
@@ -1254,6 +1459,70 @@ extern "C" int s1b_geo2rdr(const s1b_burst_plan_t *plan, const int16_t *dem, int
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr: DEM window too tall");
   geo2rdr_kernel<<<grid, G_TX, 0, st>>>(*plan, dem, dem_pitch, (const float2 *)deramped,
                                          (float2 *)out, rows, nrow, ncol, g_cull_geo != 0);
+  return s1b_launch_status();
+}
+
+extern "C" size_t s1b_geocode_scratch_bytes(const s1b_burst_plan_t *plan) {
+  return plan && plan->samples > 0 ? (size_t)plan->samples * (sizeof(double2) + sizeof(float2)) : 0;
+}
+
+extern "C" int s1b_geocode(const s1b_burst_plan_t *plan, const void *slc, int32_t sample_format, const int16_t *dem,
+                           int64_t dem_pitch, void *out, int32_t *rows, void *scratch, size_t scratch_bytes,
+                           void *stream) {
+  if (!plan || !slc || !dem || !out || !scratch)
+    return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geocode: null argument");
+  if (sample_format != S1B_SAMPLES_C64 && sample_format != S1B_SAMPLES_CI16)
+    return s1b_fail(S1B_ERR_UNSUPPORTED, "s1b_geocode: unknown sample format");
+  const int nrow = plan->win_bottom - plan->win_top, ncol = plan->win_right - plan->win_left;
+  if (nrow <= 0 || ncol <= 0) return s1b_fail(S1B_ERR_EMPTY, "s1b_geocode: empty DEM window");
+  if (plan->lines < 1 || plan->samples < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geocode: empty burst");
+  if (dem_pitch < ncol) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geocode: dem_pitch < window width");
+  if (scratch_bytes < s1b_geocode_scratch_bytes(plan) || reinterpret_cast<uintptr_t>(scratch) % 16 != 0)
+    return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geocode: scratch too small or not 16-byte aligned");
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const unsigned gx = (unsigned)((ncol + G_TX - 1) / G_TX);
+  // few tiles: short ones, so that more warps share the rows (512 x 2048
+  // samples, 162 tiles: 41 us a call with 8 rows, 52 with 32; 1500 x 4500,
+  // about 1100 tiles: 83 and 77)
+  const bool small = (int64_t)gx * ((nrow + 31) / 32) < 3 * (int64_t)sms;
+  const int ry = small ? 8 : 32;
+  const unsigned gy = (unsigned)((nrow + ry - 1) / ry);
+  if (gy > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geocode: DEM window too tall");
+  GeocodeArgs a;
+  a.dem = dem;
+  a.pitch = dem_pitch;
+  a.slc = slc;
+  double2 *tops = (double2 *)scratch;
+  float2 *slopes = (float2 *)(tops + plan->samples);
+  a.tops = tops;
+  a.slopes = slopes;
+  a.out = (float2 *)out;
+  a.rows = rows;
+  a.nrow = nrow;
+  a.ncol = ncol;
+  a.cull = g_cull_geo;
+  a.gc = geo_consts(*plan);
+  const s1b_burst_plan_t &p = *plan;
+  a.rg_first = std::max(-1, p.first_valid_sample);
+  a.rg_span = (uint32_t)std::max<int64_t>(0, std::min<int64_t>((int64_t)p.last_valid_sample - 1, p.samples - 1) - a.rg_first);
+  a.az_first = (int32_t)std::max<int64_t>(-1, (int64_t)p.first_valid_line + 5);
+  a.az_span = (uint32_t)std::max<int64_t>(0, std::min<int64_t>((int64_t)p.last_valid_line - 5, p.lines - 1) - a.az_first);
+  cudaStream_t st = (cudaStream_t)stream;
+  geocode_tables_kernel<<<(unsigned)((plan->samples + 127) / 128), 128, 0, st>>>(*plan, tops, slopes, rows, nrow);
+  int s = s1b_launch_status();
+  if (s) return s;
+  const dim3 grid(gx, gy);
+  if (sample_format == S1B_SAMPLES_CI16) {
+    if (small)
+      geocode_kernel<8, short2><<<grid, G_TX, 0, st>>>(*plan, a);
+    else
+      geocode_kernel<32, short2><<<grid, G_TX, 0, st>>>(*plan, a);
+  } else if (small) {
+    geocode_kernel<8, float2><<<grid, G_TX, 0, st>>>(*plan, a);
+  } else {
+    geocode_kernel<32, float2><<<grid, G_TX, 0, st>>>(*plan, a);
+  }
   return s1b_launch_status();
 }
 

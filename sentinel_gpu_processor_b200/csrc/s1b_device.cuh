@@ -72,6 +72,34 @@ __device__ __forceinline__ double i32_to_f64(int x) {
   return __longlong_as_double(0x4338000000000000LL + (long long)x) - 6755399441055744.0;
 }
 
+// floor(x) of |x| < 2^31 and its int, from two FP64 additions: adding 1.5 *
+// 2^52 with rounding down leaves floor(x) in the low bits.  No conversion unit.
+__device__ __forceinline__ double floor_int(double x, int &i) {
+  const double t = __dadd_rd(x, 6755399441055744.0);
+  i = __double2loint(t);
+  return t - 6755399441055744.0;
+}
+
+// Unit phasor exp(i pi h) of an FP64 phase h in half-cycles (|h| < 2^50): the
+// nearest quarter k/2 is taken off in FP64 (k from the low bits of 2 h + 1.5 *
+// 2^52), the rest, |r| <= 1/4, is rounded once (<= 1.5e-8 half-cycles) and sin
+// and cos of pi r are polynomials in r^2 that interpolate at the Chebyshev
+// nodes of [0, 1/16] (computed in extended precision): absolute error below
+// 9e-8, rms 2e-8 each.  Half the instructions of phasor_pi, none of them on
+// the conversion unit but the rounding, and a quarter of its phase rounding.
+__device__ __forceinline__ float2 phasor_quarter(double h) {
+  const double t = fma(h, 2.0, 6755399441055744.0);
+  const int k = __double2loint(t);
+  const float r = (float)fma(-0.5, t - 6755399441055744.0, h);
+  const float v = r * r;
+  const float s = r * fmaf(v, fmaf(v, fmaf(v, -5.890750992e-01f, 2.549766965e+00f), -5.167707821e+00f), 3.141592644e+00f);
+  const float c = fmaf(v, fmaf(v, fmaf(v, fmaf(v, 2.321254140e-01f, -1.335137814e+00f), 4.058710566e+00f),
+                               -4.934802197e+00f), 1.f);
+  const float x = k & 1 ? s : c, y = k & 1 ? c : s;
+  return make_float2(__int_as_float(__float_as_int(x) ^ (((k + 1) & 2) << 30)),
+                     __int_as_float(__float_as_int(y) ^ ((k & 2) << 30)));
+}
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }

@@ -37,11 +37,14 @@ def geocode_burst(plan, slc: torch.Tensor, dem: torch.Tensor, deramped: torch.Te
     if plan.nrow <= 0 or plan.ncol <= 0:
         return None
     flat = slc.reshape(-1, 2) if slc.dtype == torch.int16 else slc.reshape(-1)
-    deramped = kernels.deramp(plan, flat, out=deramped)
-    full, rows = kernels.geo2rdr(plan, dem, deramped, out=out)
+    if deramped is None:
+        full, rows = kernels.geocode(plan, flat, dem, out=out)
+    else:  # a buffer for the deramped burst: the caller keeps it
+        deramped = kernels.deramp(plan, flat, out=deramped)
+        full, rows = kernels.geo2rdr(plan, dem, deramped, out=out)
     if not sync:
         return full, rows
-    first, last = (int(v) for v in rows.cpu())
+    first, last = rows.tolist()
     if first >= plan.nrow or first == last or last < 0:
         return None
     return gslc_header(plan, first, last), full[first:last]

@@ -71,18 +71,7 @@ def geo2rdr(plan: _lib.BurstPlan, dem: torch.Tensor, deramped: torch.Tensor, out
     """
     _need_cuda(dem, deramped, out, rows)
     _c64(deramped, "deramped")
-    if dem.dtype != torch.int16:
-        raise ValueError("dem must be int16")
-    nrow, ncol = plan.nrow, plan.ncol
-    if nrow <= 0 or ncol <= 0:
-        raise _lib.S1BError(_lib.S1B_ERR_EMPTY, "geo2rdr")
-    if dem.shape == (plan.rsc_nlat, plan.rsc_nlon) and (dem.shape != (nrow, ncol) or
-                                                         (plan.win_top, plan.win_left) != (0, 0)):
-        win = dem[plan.win_top:plan.win_bottom, plan.win_left:plan.win_right]
-    else:
-        win = dem
-    if tuple(win.shape) != (nrow, ncol) or win.stride(1) != 1:
-        raise ValueError("dem does not cover the plan's window")
+    win, nrow, ncol = _dem_window(plan, dem, "geo2rdr")
     if out is None:
         out = torch.empty((nrow, ncol), dtype=torch.complex64, device=deramped.device)
     if rows is None:
@@ -90,6 +79,53 @@ def geo2rdr(plan: _lib.BurstPlan, dem: torch.Tensor, deramped: torch.Tensor, out
     lib = _lib.load()
     _lib.check(_call("geo2rdr", lib.s1b_geo2rdr, ctypes.byref(plan), _lib.dptr(win), win.stride(0), _lib.dptr(deramped),
                                _lib.dptr(out), _lib.dptr(rows), _lib.stream_ptr()), "s1b_geo2rdr")
+    return out, rows
+
+
+def _dem_window(plan: _lib.BurstPlan, dem: torch.Tensor, where: str):
+    """The plan's window of ``dem`` (the full RSC-grid DEM or the window itself) and its size."""
+    if dem.dtype != torch.int16:
+        raise ValueError("dem must be int16")
+    nrow, ncol = plan.nrow, plan.ncol
+    if nrow <= 0 or ncol <= 0:
+        raise _lib.S1BError(_lib.S1B_ERR_EMPTY, where)
+    if dem.shape == (plan.rsc_nlat, plan.rsc_nlon) and (dem.shape != (nrow, ncol) or
+                                                         (plan.win_top, plan.win_left) != (0, 0)):
+        win = dem[plan.win_top:plan.win_bottom, plan.win_left:plan.win_right]
+    else:
+        win = dem
+    if tuple(win.shape) != (nrow, ncol) or win.stride(1) != 1:
+        raise ValueError("dem does not cover the plan's window")
+    return win, nrow, ncol
+
+
+def geocode(plan: _lib.BurstPlan, slc: torch.Tensor, dem: torch.Tensor, out: torch.Tensor | None = None,
+            rows: torch.Tensor | None = None):
+    """:func:`deramp` and :func:`geo2rdr` in one, without the deramped copy
+    (``s1b_geocode``): ``slc`` are the burst's raw samples, complex64 or
+    complex int16 as int16 [..., 2].  The same results within float32
+    rounding; returns (out complex64 [nrow, ncol], rows int32 [2])."""
+    _need_cuda(slc, dem, out, rows)
+    ci16 = slc.dtype == torch.int16
+    if ci16:
+        if not slc.is_contiguous() or slc.shape[-1] != 2:
+            raise ValueError("int16 slc must be a contiguous [..., 2] (re, im) tensor")
+    else:
+        _c64(slc, "slc")
+    if slc.numel() != plan.lines * plan.samples * (2 if ci16 else 1):
+        raise ValueError("slc size does not match the plan")
+    win, nrow, ncol = _dem_window(plan, dem, "geocode")
+    dev = slc.device
+    if out is None:
+        out = torch.empty((nrow, ncol), dtype=torch.complex64, device=dev)
+    if rows is None:
+        rows = torch.empty(2, dtype=torch.int32, device=dev)
+    lib = _lib.load()
+    need = 24 * plan.samples  # s1b_geocode_scratch_bytes
+    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    _lib.check(_call("geocode", lib.s1b_geocode, ctypes.byref(plan), _lib.dptr(slc),
+                     _lib.S1B_SAMPLES_CI16 if ci16 else _lib.S1B_SAMPLES_C64, _lib.dptr(win), win.stride(0),
+                     _lib.dptr(out), _lib.dptr(rows), _lib.dptr(scratch), need, _lib.stream_ptr()), "s1b_geocode")
     return out, rows
 
 
