@@ -26,25 +26,76 @@ namespace {
 constexpr double kRaD = 6378137.0;
 constexpr double kRe2D = 0.00669437999015;
 
-// -------------------------------------------------------------- offsets
-// Same column walk as the geocoding kernel: thread = reference column, 16
-// rows per thread; the first row solves on the window polynomial from the
-// burst centre, the others on the cubic expansion there (OrbitCubic).
-constexpr int O_TX = 128, O_RY = 16;
-
-// ECEF position of a geodetic point and the geodetic up vector dp/dh.
-__device__ __forceinline__ void llh_ecef(double lat_deg, double lon_deg, double h, double p[3], double up[3]) {
-  double sl, cl, so, co;
-  sincospi(lat_deg * (1.0 / 180.0), &sl, &cl);
-  sincospi(lon_deg * (1.0 / 180.0), &so, &co);
-  const double re = kRaD * rsqrt(1. - kRe2D * sl * sl);  // orbit.cu:27-30
-  p[0] = (re + h) * cl * co;
-  p[1] = (re + h) * cl * so;
-  p[2] = (re * (1 - kRe2D) + h) * sl;
-  up[0] = cl * co;
-  up[1] = cl * so;
-  up[2] = sl;
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
 }
+
+// -------------------------------------------------------------- offsets
+// Thread = reference column, O_RY rows; one orbit patch per warp (32 columns x
+// O_RY rows, ZeroDopplerPatch) about the zero-Doppler time of its centre pixel.
+// What bounds it is the FP64 pipe, so a pixel's FP64 operations are what was
+// cut, from about 210 to 85:
+//   * sines and cosines of latitude and longitude and the prime vertical
+//     radius come by Taylor series from the column's last full evaluation
+//     (PointBase);
+//   * four dot products on the patch, one Newton step with a refined slope from
+//     the row's own time (a second where the first is above 1e-4 s), and the
+//     range from the same coefficients, instead of two orbit evaluations with
+//     a division each; no row waits for the one above.
+// A pixel off the patch (more than 0.25 s from its centre, or a second step
+// above 1e-6 s) is solved on the orbit polynomials.  The inputs stream through
+// a ring of O_AHEAD rows in shared memory by cp.async (a lane reads back only
+// what it copied itself: no barrier); one row ahead in registers left the FP64
+// pipe waiting for DRAM.  1500 x 21000: 443 -> 288 us (FP64 pipe 49 % busy,
+// its latency filled by 16 warps per SM and two rows each; 5 CTAs at 96
+// registers spill: 358; 32 rows per CTA 309, 128 rows 292).
+constexpr int O_TX = 128, O_RY = 64, O_AHEAD = 8;
+
+// |x| > limit (or x no number), by the high words: off the FP64 pipe.
+__device__ __forceinline__ bool above(double x, double limit) {
+  return (__double2hiint(x) & 0x7fffffff) > __double2hiint(limit);
+}
+
+// Geodetic point (degrees, metres) to ECEF near a point evaluated in full,
+// orbit.cu:27-30.  With both angles within 1e-4 rad of the base's, sin x = x -
+// x^3 / 6 and cos x - 1 = -x^2 / 2 are exact to 1e-17, and with d = (y - y0) /
+// (1 - y0), y = e^2 sin^2 lat (|d| < 2e-6), the prime vertical radius re0
+// (1 - d)^-1/2 = re0 (1 + d / 2 + 3 d^2 / 8) to 1e-17.  Beyond, the point
+// becomes the new base.
+struct PointBase {
+  double lat, lon, sl, cl, so, co, re, ki, k0;
+  __device__ __forceinline__ void full(double la, double lo) {
+    lat = la;
+    lon = lo;
+    sincospi(la * (1.0 / 180.0), &sl, &cl);
+    sincospi(lo * (1.0 / 180.0), &so, &co);
+    const double y = kRe2D * sl * sl, i = 1.0 / (1.0 - y);
+    re = kRaD * rsqrt(1.0 - y);
+    ki = kRe2D * i;
+    k0 = y * i;
+  }
+  // p, and sine and cosine of its latitude (up[0], up[1]) and longitude (up[2], up[3])
+  __device__ __forceinline__ void ecef(double la, double lo, double h, double p[3], double up[4]) {
+    double x = (la - lat) * (kPiD / 180.0), y = (lo - lon) * (kPiD / 180.0);
+    if (above(x, 1.0e-4) || above(y, 1.0e-4)) {
+      full(la, lo);
+      x = y = 0.0;
+    }
+    const double x2 = x * x, y2 = y * y;
+    const double sx = fma(x * x2, -1.0 / 6.0, x), sy = fma(y * y2, -1.0 / 6.0, y);
+    const double s = fma(-0.5 * sl, x2, fma(cl, sx, sl)), c = fma(-0.5 * cl, x2, fma(-sl, sx, cl));
+    const double so1 = fma(-0.5 * so, y2, fma(co, sy, so)), co1 = fma(-0.5 * co, y2, fma(-so, sy, co));
+    const double d = fma(s * s, ki, -k0);
+    const double r = fma(re * d, fma(0.375, d, 0.5), re), rho = (r + h) * c;
+    p[0] = rho * co1;
+    p[1] = rho * so1;
+    p[2] = fma(r, 1 - kRe2D, h) * s;
+    up[0] = s;
+    up[1] = c;
+    up[2] = so1;
+    up[3] = co1;
+  }
+};
 
 // Height sensitivity of the secondary offsets of a reference-grid pixel.  A
 // height error moves the ground point along the reference's zero-Doppler
@@ -52,7 +103,7 @@ __device__ __forceinline__ void llh_ecef(double lat_deg, double lon_deg, double 
 // (range to and Doppler of the reference unchanged, geodetic height +1).
 // The secondary then sees f(t, p) = (p - X(t)).V(t) = 0 move by dt/dh =
 // (V.dp) / (|V|^2 - dr.A) and its range by rhat.(dp - V dt/dh).
-__device__ __forceinline__ void height_sensitivity(const OrbitCubic &o, double t, const double dr[3],
+__device__ __forceinline__ void height_sensitivity(const double v[3], const double a[3], const double dr[3],
                                                    const double up[3], const double rr[3], const double vr[3],
                                                    double &dt_dh, double &dR_dh) {
   // c = dr_ref x V_ref (the unit of dr_ref cancels in the ratio)
@@ -61,13 +112,6 @@ __device__ __forceinline__ void height_sensitivity(const OrbitCubic &o, double t
   const double c2 = rr[0] * vr[1] - rr[1] * vr[0];
   const double inv = 1.0 / (up[0] * c0 + up[1] * c1 + up[2] * c2);
   const double dp[3] = {c0 * inv, c1 * inv, c2 * inv};
-  const double h = t - o.t0;
-  double v[3], a[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    a[i] = fma(o.j[i], h, o.a[i]);
-    v[i] = fma(fma(0.5 * o.j[i], h, o.a[i]), h, o.v[i]);
-  }
   const double vn = v[0] * dp[0] + v[1] * dp[1] + v[2] * dp[2];
   const double den = (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) - (dr[0] * a[0] + dr[1] * a[1] + dr[2] * a[2]);
   dt_dh = vn / den;
@@ -84,7 +128,7 @@ struct RefOrbit {
 };
 
 template <bool kSens>
-__global__ __launch_bounds__(O_TX) void offsets_kernel(const __grid_constant__ s1b_burst_plan_t P,
+__global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant__ s1b_burst_plan_t P,
                                                        const __grid_constant__ RefOrbit R,
                                                        const double *__restrict__ lat,
                                                        const double *__restrict__ lon,
@@ -93,17 +137,23 @@ __global__ __launch_bounds__(O_TX) void offsets_kernel(const __grid_constant__ s
                                                        float *__restrict__ rg_off,
                                                        float *__restrict__ daz_dh,
                                                        float *__restrict__ drg_dh) {
-  const int col = blockIdx.x * O_TX + threadIdx.x;
+  __shared__ double s_in[O_AHEAD][3][O_TX];
+  static_assert((O_AHEAD & (O_AHEAD - 1)) == 0, "ring slots are taken modulo a power of two");
+  // the last block's spare lanes repeat the last column
+  const int col = min((int)(blockIdx.x * O_TX + threadIdx.x), S - 1);
+  const bool store = blockIdx.x * O_TX + threadIdx.x < S;
   const int row0 = blockIdx.y * O_RY;
-  if (col >= S) return;
-  const double inv_dmrg = 1.0 / P.dmrg, prf = 1.0 / P.dtaz;
+  const double inv_dmrg = 1.0 / P.dmrg, prf = 1.0 / P.dtaz, cold = col;
   const int rmax = min(O_RY, L - row0);
-  size_t i = (size_t)row0 * S + col;
-  double la = __ldcs(lat + i), lo = __ldcs(lon + i), h = __ldcs(hgt + i);
-  double p[3], dr[3], up[3];
-  // first row: from the burst centre on the window polynomial
-  double t = P.tmid;
-  {
+  ZeroDopplerPatch z;
+  {  // the warp's centre pixel on the orbit polynomials (the same in every lane)
+    const int cw = min((int)(blockIdx.x * O_TX + (threadIdx.x & ~31) + 16), S - 1);
+    const size_t i = (size_t)(row0 + rmax / 2) * S + cw;
+    PointBase base;
+    double p[3], up[4], dr[3];
+    base.full(__ldg(lat + i), __ldg(lon + i));
+    base.ecef(base.lat, base.lon, __ldg(hgt + i), p, up);
+    double t = P.tmid;
     OrbitState st;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -111,45 +161,106 @@ __global__ __launch_bounds__(O_TX) void offsets_kernel(const __grid_constant__ s
       st.v[k] = P.vmid[k];
       st.a[k] = P.amid[k];
     }
-    llh_ecef(la, lo, h, p, up);
     zero_doppler(P.orbit, p, t, st, dr);
-  }
-  OrbitCubic o;
-  orbit_cubic(P.orbit, t, o);
-  double tprev = t - P.dtaz;
-  // the next row's inputs are loaded one row ahead
-  if (rmax > 1) {
-    la = __ldcs(lat + i + S);
-    lo = __ldcs(lon + i + S);
-    h = __ldcs(hgt + i + S);
-  }
-  for (int r = 0;;) {
-    const double rng = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-    // residuals relative to the pixel index keep float32 at ~1e-5 px
-    __stcs(az_off + i, (float)((t - P.tstart) * prf - (row0 + r)));
-    __stcs(rg_off + i, (float)((rng - P.rngstart) * inv_dmrg - col));
-    if (kSens) {
-      OrbitState rs;
-      orbit_eval(R.orbit, R.tstart + (row0 + r) * R.dtaz, rs);
-      const double rr[3] = {p[0] - rs.x[0], p[1] - rs.x[1], p[2] - rs.x[2]};
-      double dt_dh, dR_dh;
-      height_sensitivity(o, t, dr, up, rr, rs.v, dt_dh, dR_dh);
-      __stcs(daz_dh + i, (float)(dt_dh * prf));
-      __stcs(drg_dh + i, (float)(dR_dh * inv_dmrg));
+    OrbitCubic o;
+    orbit_cubic(P.orbit, t, o);
+    zero_doppler_patch(o, z);
+    z.inv_c1 = 1.0 / zero_doppler_point(z, p).c1;
+    // the patch's rows reach 0.07 s from its centre, where the velocity's h^3
+    // term, left out of ZeroDopplerPatch, moves the root by 8e-13 s: its
+    // product with the centre's line of sight joins c3
+    const int w = s1b_orbit_window(P.orbit, t) - 1;
+    const double tau = t - P.orbit.tc[w];
+    double ds = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double *c = P.orbit.c[w][k];
+      const double snap = fma(fma(fma(840.0 * c[7], tau, 360.0 * c[6]), tau, 120.0 * c[5]), tau, 24.0 * c[4]);
+      ds = fma(p[k] - z.x[k], snap, ds);
     }
-    if (++r >= rmax) break;
+    z.c3 = fma(ds, 1.0 / 6.0, z.c3);
+  }
+  size_t i = (size_t)row0 * S + col;
+  size_t inext = i;  // pixel of the next row to copy
+  int copied = 0;
+  auto copy_rows = [&]() {  // one group of two rows
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (copied < rmax) {
+        double(*slot)[O_TX] = s_in[copied & (O_AHEAD - 1)];
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(&slot[0][threadIdx.x])), "l"(lat + inext));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(&slot[1][threadIdx.x])), "l"(lon + inext));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(&slot[2][threadIdx.x])), "l"(hgt + inext));
+        inext += S;
+        ++copied;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < O_AHEAD / 2 - 1; ++k) copy_rows();
+  PointBase base;
+  base.full(__ldg(lat + i), __ldg(lon + i));
+  double rowd = row0;
+  double hseed = -(rmax / 2) * P.dtaz;  // time of the row from the patch's
+  // two rows at a time, so that one's FP64 chain fills the other's gaps
+  for (int r0 = 0; r0 < rmax; r0 += 2) {
+  double in[2][3];
+  asm volatile("cp.async.wait_group %0;" ::"n"(O_AHEAD / 2 - 2) : "memory");  // this lane's copies of both have landed
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) in[k][c] = s_in[(r0 + (r0 + k < rmax ? k : 0)) & (O_AHEAD - 1)][c][threadIdx.x];
+  copy_rows();  // into the slots of the two rows before
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    double p[3], up[4];
+    base.ecef(in[k][0], in[k][1], in[k][2], p, up);
+    const ZeroDopplerPoint q = zero_doppler_point(z, p);
+    // seed: the row's own time (the secondary sees it there within ~1e-5 s)
+    double hn = hseed;
+    hseed += P.dtaz;
+    const double slope = fma(2.0 * q.c2, hn, q.c1);
+    const double inv = z.inv_c1 * fma(-slope, z.inv_c1, 2.0);  // 1 / f' to 1e-7 or better
+    double step = inv * fma(fma(fma(z.c3, hn, q.c2), hn, q.c1), hn, q.c0);
+    hn -= step;
+    bool on_patch = !above(hn, 0.25);
+    if (above(step, 1.0e-4)) {
+      step = inv * fma(fma(fma(z.c3, hn, q.c2), hn, q.c1), hn, q.c0);
+      hn -= step;
+      on_patch = !above(hn, 0.25) && !above(step, 1.0e-6);
+    }
+    double rng;
+    if (on_patch) {
+      rng = sqrt_heron(fma(-hn, fma(fma(fma(0.5 * z.c3, hn, (2.0 / 3.0) * q.c2), hn, q.c1), hn, 2.0 * q.c0), q.dd));
+    } else {
+      OrbitState st;
+      double t = P.tmid, dr[3];
+      orbit_eval(P.orbit, t, st);
+      zero_doppler(P.orbit, p, t, st, dr);
+      rng = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
+      hn = t - z.t0;
+    }
+    if (store && r0 + k < rmax) {
+      // residuals relative to the pixel index keep float32 at ~1e-5 px
+      __stcs(az_off + i, (float)((z.t0 + hn - P.tstart) * prf - rowd));
+      __stcs(rg_off + i, (float)fma(rng - P.rngstart, inv_dmrg, -cold));
+      if (kSens) {
+        OrbitState rs, st;
+        orbit_eval(R.orbit, R.tstart + rowd * R.dtaz, rs);
+        orbit_eval(P.orbit, z.t0 + hn, st);
+        const double n[3] = {up[1] * up[3], up[1] * up[2], up[0]};
+        const double rr[3] = {p[0] - rs.x[0], p[1] - rs.x[1], p[2] - rs.x[2]};
+        const double dr[3] = {p[0] - st.x[0], p[1] - st.x[1], p[2] - st.x[2]};
+        double dt_dh, dR_dh;
+        height_sensitivity(st.v, st.a, dr, n, rr, rs.v, dt_dh, dR_dh);
+        __stcs(daz_dh + i, (float)(dt_dh * prf));
+        __stcs(drg_dh + i, (float)(dR_dh * inv_dmrg));
+      }
+    }
+    rowd += 1.0;
     i += S;
-    llh_ecef(la, lo, h, p, up);
-    if (r + 1 < rmax) {
-      la = __ldcs(lat + i + S);
-      lo = __ldcs(lon + i + S);
-      h = __ldcs(hgt + i + S);
-    }
-    // seed: linear extrapolation down the column
-    const double tn = 2.0 * t - tprev;
-    tprev = t;
-    t = tn;
-    zero_doppler_cubic(o, p, t, dr);
+  }
   }
 }
 
@@ -157,10 +268,6 @@ __global__ __launch_bounds__(O_TX) void offsets_kernel(const __grid_constant__ s
 // Bounded wait: try_wait suspends for a hardware time slice per call; after
 // kSpinLimit calls the caller treats the copy as lost.
 constexpr uint32_t kSpinLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = kSpinLimit) {
   for (uint32_t i = 0; i < limit; ++i) {

@@ -168,11 +168,9 @@ __device__ __forceinline__ int zero_doppler(const s1b_orbit_poly_t &P, const dou
 }
 
 // Cubic expansion of the orbit about t0 (position, velocity, acceleration,
-// jerk of the window polynomial).  A column walk solves its first pixel on
-// the polynomial and the following ones on the expansion: over a segment of
-// 16 lines (|t - t0| <= ~0.035 s) the dropped fourth-order term is
-// snap |dt|^4 / 24 < 1e-12 m for an orbit (snap ~ omega^4 r ~ 1e-5 m/s^4),
-// and each Newton step costs 18 FMA instead of a 54-FMA polynomial pass.
+// jerk of the window polynomial), from which a patch of pixels is solved
+// (ZeroDopplerPatch): within 0.035 s the dropped fourth-order term is snap
+// |dt|^4 / 24 < 1e-12 m for an orbit (snap ~ omega^4 r ~ 1e-5 m/s^4).
 struct OrbitCubic {
   double t0, x[3], v[3], a[3], j[3];
 };
@@ -197,32 +195,6 @@ __device__ __forceinline__ void orbit_cubic(const s1b_orbit_poly_t &P, double t,
     o.v[comp] = d;
     o.a[comp] = 2.0 * dd;
     o.j[comp] = 6.0 * ddd;
-  }
-}
-
-// Zero-Doppler Newton (same iteration and stopping rule as zero_doppler)
-// with the orbit state taken from the cubic expansion.
-__device__ __forceinline__ void zero_doppler_cubic(const OrbitCubic &o, const double p[3], double &t, double dr[3]) {
-  for (int it = 0; it < 51; ++it) {
-    const double h = t - o.t0;
-    double fn = 0.0, fp = 0.0, v[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double a = fma(o.j[i], h, o.a[i]);
-      v[i] = fma(fma(0.5 * o.j[i], h, o.a[i]), h, o.v[i]);
-      const double x = fma(fma(fma(o.j[i] * (1.0 / 6.0), h, 0.5 * o.a[i]), h, o.v[i]), h, o.x[i]);
-      dr[i] = p[i] - x;
-      fn = fma(dr[i], v[i], fn);
-      fp = fma(dr[i], a, fp);
-      fp = fma(-v[i], v[i], fp);
-    }
-    const double step = fn / fp;
-    t -= step;
-    if (fabs(step) < 5.0e-9) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) dr[i] = fma(step, v[i], dr[i]);
-      return;
-    }
   }
 }
 
@@ -357,29 +329,6 @@ __device__ __forceinline__ double rcp_newton(double x) {
   double r = (double)__fdividef(1.0f, (float)x);
   r = fma(r, fma(-x, r, 1.0), r);
   return fma(r, fma(-x, r, 1.0), r);
-}
-
-// zero_doppler_cubic with a fixed reciprocal derivative (chord Newton).
-__device__ __forceinline__ void zero_doppler_cubic_chord(const OrbitCubic &o, const double p[3], double &t,
-                                                         double dr[3], double inv_fp) {
-  for (int it = 0; it < 51; ++it) {
-    const double h = t - o.t0;
-    double fn = 0.0, v[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      v[i] = fma(fma(0.5 * o.j[i], h, o.a[i]), h, o.v[i]);
-      const double x = fma(fma(fma(o.j[i] * (1.0 / 6.0), h, 0.5 * o.a[i]), h, o.v[i]), h, o.x[i]);
-      dr[i] = p[i] - x;
-      fn = fma(dr[i], v[i], fn);
-    }
-    const double step = fn * inv_fp;
-    t -= step;
-    if (fabs(step) < 5.0e-9) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) dr[i] = fma(step, v[i], dr[i]);
-      return;
-    }
-  }
 }
 
 // One full-resolution pixel pair into the multilook sums of crossmul:
