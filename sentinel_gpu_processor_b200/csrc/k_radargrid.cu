@@ -20,6 +20,7 @@
 #include "s1b.h"
 #include "s1b_device.cuh"
 #include "s1b_internal.h"
+#include "s1b_sinc.cuh"
 
 namespace {
 
@@ -294,56 +295,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 constexpr int R_TX = 64, R_TY = 4, R_RPT = 4;  // columns, row groups, rows per thread
 constexpr int R_TH = R_TY * R_RPT;             // 16 tile rows
 constexpr int R_WROWS = 32, R_WCOLS = 96;
-constexpr int SINC_BINS = 1024;
-
-// Normalised 8-tap windowed-sinc weights at SINC_BINS + 1 fractions f = b /
-// SINC_BINS (taps k = -3..4 at distance k - f: sinc(k - f) (0.5 + 0.5
-// cos(pi (k - f) / 4)), divided by their sum); evaluated by the host in
-// double precision, read with linear interpolation in the fraction.
-__device__ __align__(16) float g_sinc_table[(SINC_BINS + 1) * 8];
-std::mutex g_sinc_mu;
-bool g_sinc_ready[64] = {};
-
-int ensure_sinc_table() {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e));
-  if (dev < 0 || dev >= 64) return s1b_fail(S1B_ERR_UNSUPPORTED, "s1b_resample: device ordinal above 63");
-  std::lock_guard<std::mutex> lock(g_sinc_mu);
-  if (g_sinc_ready[dev]) return S1B_OK;
-  static float host[(SINC_BINS + 1) * 8];
-  for (int b = 0; b <= SINC_BINS; ++b) {
-    const double f = (double)b / SINC_BINS;
-    double w[8], sum = 0.0;
-    for (int k = 0; k < 8; ++k) {
-      const double x = (k - 3) - f;
-      const double sc = x == 0.0 ? 1.0 : sin(kPiD * x) / (kPiD * x);
-      w[k] = sc * (0.5 + 0.5 * cos(kPiD * x / 4.0));
-      sum += w[k];
-    }
-    for (int k = 0; k < 8; ++k) host[b * 8 + k] = (float)(w[k] / sum);
-  }
-  e = cudaMemcpyToSymbol(g_sinc_table, host, sizeof(host));
-  if (e != cudaSuccess) return s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e));
-  g_sinc_ready[dev] = true;
-  return S1B_OK;
-}
-
-__device__ __forceinline__ void sinc8_weights(float f, float w[8]) {
-  const float pos = f * SINC_BINS;
-  const int b = min((int)pos, SINC_BINS - 1);
-  const float t = pos - (float)b;
-  const float4 *T = reinterpret_cast<const float4 *>(g_sinc_table) + 2 * b;
-  const float4 a0 = __ldg(T), a1 = __ldg(T + 1), b0 = __ldg(T + 2), b1 = __ldg(T + 3);
-  w[0] = fmaf(t, b0.x - a0.x, a0.x);
-  w[1] = fmaf(t, b0.y - a0.y, a0.y);
-  w[2] = fmaf(t, b0.z - a0.z, a0.z);
-  w[3] = fmaf(t, b0.w - a0.w, a0.w);
-  w[4] = fmaf(t, b1.x - a1.x, a1.x);
-  w[5] = fmaf(t, b1.y - a1.y, a1.y);
-  w[6] = fmaf(t, b1.z - a1.z, a1.z);
-  w[7] = fmaf(t, b1.w - a1.w, a1.w);
-}
 
 // TOPS coefficients at a continuous range sample, the phase in half-cycles
 // (units of pi rad): -kt, so that the deramp phase is pi (-kt) (eta -
@@ -382,22 +333,38 @@ struct Coord {
   bool ok;
 };
 
-__device__ __forceinline__ Coord coord_of(const s1b_burst_plan_t &P, const float *az_off, const float *rg_off,
-                                          int row, int col, int S, int lo, int hi) {
+// floor(a) of |a| < 2^22 as float and int: adding 1.5 * 2^23 with rounding down
+// leaves it in the low bits, off the conversion unit.
+__device__ __forceinline__ float floor_small(float a, int &i) {
+  const float t = __fadd_rd(a, 12582912.f);
+  i = __float_as_int(t) - 0x4B400000;
+  return t - 12582912.f;
+}
+
+// From the offsets (a, r) of output (row, col); `in`: it is part of the raster.
+__device__ __forceinline__ Coord coord_from(const s1b_burst_plan_t &P, float a, float r, int row, int col, bool in,
+                                            int lo, int hi) {
   Coord k;
-  const size_t i = (size_t)row * S + col;
-  const float a = __ldg(az_off + i), r = __ldg(rg_off + i);
   // offsets of 2^20 samples or more (and NaN) leave any burst
-  k.ok = fabsf(a) < 0x1p20f && fabsf(r) < 0x1p20f;
-  const float fla = k.ok ? floorf(a) : 0.f, flr = k.ok ? floorf(r) : 0.f;
-  k.na = row + (int)fla;
-  k.nr = col + (int)flr;
+  k.ok = in && fabsf(a) < 0x1p20f && fabsf(r) < 0x1p20f;
+  int ia, ir;
+  const float fla = floor_small(a, ia), flr = floor_small(r, ir);
+  k.na = row + ia;
+  k.nr = col + ir;
   // a - floor(a) is exact for a >= 0; for a small negative a it can round
   // to 1.0f, which would put a sinc tap at distance 0 from the wrong sample
   k.fa = fminf(a - fla, 0x1.fffffep-1f);
   k.fr = fminf(r - flr, 0x1.fffffep-1f);
-  k.ok = k.ok && k.na - lo >= 0 && k.na + hi < P.lines && k.nr - lo >= 0 && k.nr + hi < P.samples;
+  // n - lo >= 0 and n + hi < size
+  k.ok = k.ok && (unsigned)(k.na - lo) < (unsigned)max(0, P.lines - lo - hi) &&
+         (unsigned)(k.nr - lo) < (unsigned)max(0, P.samples - lo - hi);
   return k;
+}
+
+__device__ __forceinline__ Coord coord_of(const s1b_burst_plan_t &P, const float *az_off, const float *rg_off,
+                                          int row, int col, int S, int lo, int hi) {
+  const size_t i = (size_t)row * S + col;
+  return coord_from(P, __ldg(az_off + i), __ldg(rg_off + i), row, col, true, lo, hi);
 }
 
 // Restore the secondary's TOPS phase at the fractional position (az lines).
@@ -601,12 +568,19 @@ __global__ __launch_bounds__(R_TX *R_TY, 2) void resample_kernel(const __grid_co
 //              one of three stages;
 //   window   - the raw secondary window of the tile, box RT_WC x RT_WR at an
 //              even column (16-byte rule), issued one tile ahead into one of
-//              two stages as soon as the tile's coordinate range is known;
-//   sinc LUT - copied once per CTA.
+//              two stages as soon as the tile's coordinate range is known.
 // Per tile the CTA (1) reduces the next tile's coordinate range and issues
 // its window, (2) deramps the current window in place, (3) interpolates,
 // reramps and stores.  Waits are bounded; a wait that runs out sets *status,
 // lets the copies in flight land (again bounded) and ends the block.
+//
+// Bound by instruction issue (about 390 a pixel, 144 of them the 8 x 8 taps'
+// FFMA and FFMA2) with two CTAs of 128 registers a thread; its 756 MB would take
+// 115 us.  The weights are polynomials and not a table in shared memory: eight
+// 128-bit gathers a pixel at 64 different fractions a warp were half of the
+// shared-memory wavefronts.  1500 x 21000 samples: 711 us with the table, 635
+// with the polynomials, 602 with floors off the conversion unit, one redux for
+// the CTA's coordinate range and quarter-turn phasors.
 constexpr int RT_THREADS = R_TX * R_TY;           // 256: 64 columns x 4 row groups of 4 rows
 constexpr int RT_WR = 32, RT_WC = 96;             // window box rows x columns
 constexpr int RT_OFF_BYTES = 2 * R_TH * R_TX * 4; // az + rg blocks of one tile
@@ -615,40 +589,10 @@ constexpr int RT_WIN_BYTES = RT_WR * RT_WC * 8;
 struct RtSmem {
   float2 win[2][RT_WR][RT_WC];
   float offs[3][2][R_TH][R_TX];
-  float lut[(SINC_BINS + 1) * 8];
   double mkt[2][RT_WC], eref[2][RT_WC];  // per window stage
-  int red[RT_THREADS / 32][4];
+  int4 red[RT_THREADS / 32];
   uint64_t bar_off[3], bar_win[2];
 };
-
-__device__ __forceinline__ void sinc8_weights_lut(const float *lut, float f, float w[8]) {
-  const float pos = f * SINC_BINS;
-  const int b = min((int)pos, SINC_BINS - 1);
-  const float t = pos - (float)b;
-  const float4 *T = reinterpret_cast<const float4 *>(lut) + 2 * b;
-  const float4 a0 = T[0], a1 = T[1], b0 = T[2], b1 = T[3];
-  const float2 tt = make_float2(t, t), m1 = make_float2(-1.f, -1.f);
-  const float2 w01 = __ffma2_rn(tt, __ffma2_rn(m1, make_float2(a0.x, a0.y), make_float2(b0.x, b0.y)), make_float2(a0.x, a0.y));
-  const float2 w23 = __ffma2_rn(tt, __ffma2_rn(m1, make_float2(a0.z, a0.w), make_float2(b0.z, b0.w)), make_float2(a0.z, a0.w));
-  const float2 w45 = __ffma2_rn(tt, __ffma2_rn(m1, make_float2(a1.x, a1.y), make_float2(b1.x, b1.y)), make_float2(a1.x, a1.y));
-  const float2 w67 = __ffma2_rn(tt, __ffma2_rn(m1, make_float2(a1.z, a1.w), make_float2(b1.z, b1.w)), make_float2(a1.z, a1.w));
-  w[0] = w01.x; w[1] = w01.y; w[2] = w23.x; w[3] = w23.y;
-  w[4] = w45.x; w[5] = w45.y; w[6] = w67.x; w[7] = w67.y;
-}
-
-// Coordinate of one output from its offsets (as coord_of, values given).
-__device__ __forceinline__ Coord coord_from(const s1b_burst_plan_t &P, float a, float r, int row, int col, bool in,
-                                            int lo, int hi) {
-  Coord k;
-  k.ok = in && fabsf(a) < 0x1p20f && fabsf(r) < 0x1p20f;
-  const float fla = k.ok ? floorf(a) : 0.f, flr = k.ok ? floorf(r) : 0.f;
-  k.na = row + (int)fla;
-  k.nr = col + (int)flr;
-  k.fa = fminf(a - fla, 0x1.fffffep-1f);
-  k.fr = fminf(r - flr, 0x1.fffffep-1f);
-  k.ok = k.ok && k.na - lo >= 0 && k.na + hi < P.lines && k.nr - lo >= 0 && k.nr + hi < P.samples;
-  return k;
-}
 
 // Secondary window of a tile: origin (row wa0, even column wr0) and extent.
 struct Window {
@@ -684,11 +628,6 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
   const double eta0 = -P.lines * P.ati / 2.;  // line 0 from the burst centre
   const int n = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (n == 0) return;
-  {
-    const float4 *g = reinterpret_cast<const float4 *>(g_sinc_table);
-    float4 *s = reinterpret_cast<float4 *>(sm.lut);
-    for (int i = tid; i < (SINC_BINS + 1) * 2; i += RT_THREADS) s[i] = g[i];
-  }
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&sm.bar_off[i]);
     for (int i = 0; i < 2; ++i) mbar_init(&sm.bar_win[i]);
@@ -757,23 +696,16 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
     xna = __reduce_max_sync(0xffffffffu, xna);
     mnr = __reduce_min_sync(0xffffffffu, mnr);
     xnr = __reduce_max_sync(0xffffffffu, xnr);
-    if (lane == 0) {
-      sm.red[warp][0] = mna;
-      sm.red[warp][1] = xna;
-      sm.red[warp][2] = mnr;
-      sm.red[warp][3] = xnr;
-    }
+    if (lane == 0) sm.red[warp] = make_int4(mna, xna, mnr, xnr);
     // generic-proxy writes to the stages that the copies below overwrite are
     // ordered before them by this fence and the barrier
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (__syncthreads_or(!ok_wait)) return false;
-#pragma unroll
-    for (int i = 0; i < RT_THREADS / 32; ++i) {
-      mna = min(mna, sm.red[i][0]);
-      xna = max(xna, sm.red[i][1]);
-      mnr = min(mnr, sm.red[i][2]);
-      xnr = max(xnr, sm.red[i][3]);
-    }
+    const int4 all = sm.red[lane & (RT_THREADS / 32 - 1)];
+    mna = __reduce_min_sync(0xffffffffu, all.x);
+    xna = __reduce_max_sync(0xffffffffu, all.y);
+    mnr = __reduce_min_sync(0xffffffffu, all.z);
+    xnr = __reduce_max_sync(0xffffffffu, all.w);
     w = Window{0, 0, 0, 0, false};
     if (mna <= xna) {
       w.wa0 = mna - lo;
@@ -833,9 +765,9 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
         const int r0 = g * seg, r1 = min(cur.nwr, r0 + seg);
         if (r0 < r1) {
           const double u = fma((double)(cur.wa0 + r0), P.ati, -P.lines * P.ati / 2.) - eref;
-          float2 ph = phasor_pi(mkt * u * u);
-          float2 step = phasor_pi(mkt * P.ati * (2.0 * u + P.ati));
-          const float2 dstep = phasor_pi(2.0 * mkt * P.ati * P.ati);
+          float2 ph = phasor_quarter(mkt * u * u);
+          float2 step = phasor_quarter(mkt * P.ati * (2.0 * u + P.ati));
+          const float2 dstep = phasor_quarter(2.0 * mkt * P.ati * P.ati);
 #pragma unroll 4
           for (int r = r0; r < r1; ++r) {
             sm.win[s][r][c] = cmul(sm.win[s][r][c], ph);
@@ -864,8 +796,8 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
 #pragma unroll
       for (int q = 0; q < R_RPT; ++q) {
         acc[q] = make_float2(0.f, 0.f);
-        sinc8_weights_lut(sm.lut, k[q].fr, wr[q]);
-        sinc8_weights_lut(sm.lut, k[q].fa, wa[q]);
+        sinc8_weights(k[q].fr, wr[q]);
+        sinc8_weights(k[q].fa, wa[q]);
       }
       const float2 *base = &sm.win[s][k[0].na - 3 - cur.wa0][k[0].nr - 3 - cur.wr0];
 #pragma unroll
@@ -903,8 +835,8 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
           float2 acc = make_float2(0.f, 0.f);
           if (sinc) {
             float wr[8], wa[8];
-            sinc8_weights_lut(sm.lut, kq.fr, wr);
-            sinc8_weights_lut(sm.lut, kq.fa, wa);
+            sinc8_weights(kq.fr, wr);
+            sinc8_weights(kq.fa, wa);
             if (cur.staged) {
               const float2 *base = &sm.win[s][kq.na - 3 - cur.wa0][kq.nr - 3 - cur.wr0];
 #pragma unroll
@@ -1499,8 +1431,6 @@ extern "C" int s1b_resample(const s1b_burst_plan_t *plan, const void *sec, const
     return s1b_fail(S1B_ERR_UNSUPPORTED, "s1b_resample: interp must be S1B_INTERP_BILINEAR or S1B_INTERP_SINC8");
   if (lines < 1 || samples < 1 || plan->lines < 2 || plan->samples < 2)
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_resample: empty grid");
-  int s = ensure_sinc_table();
-  if (s) return s;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e));

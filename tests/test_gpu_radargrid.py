@@ -85,6 +85,24 @@ def test_resample_pipeline_matches_oracle(cuda, scene_c0):
     assert phase_rms(got, want, ok) < 1e-3
 
 
+@pytest.mark.parametrize("cols", [320, 318])  # TMA kernel, plain-load kernel
+@pytest.mark.parametrize("v", [0.0, -0.0, -1e-9, 0.99999994, -3.5, 2.0**20, -(2.0**23) - 1, np.inf, np.nan])
+def test_resample_offset_extremes(cuda, scene, cols, v):
+    """Whole, nearly whole, huge and non-finite offsets: the floor and the
+    range checks of the coordinates agree with the oracle's (tolerance of the
+    other cases: 1 - 2^-24 stands for the largest fraction, 1.2e-7 px)."""
+    pl = _plan(scene.sec)
+    sec = scene.sec_slc.to(cuda)
+    az = torch.full((scene.lat.shape[0], cols), v, dtype=torch.float32, device=cuda)
+    got = kernels.resample(pl, sec, az, az).cpu().numpy()
+    if not abs(v) < 2.0**20:
+        assert not got.any()
+        return
+    want, ok = _oracle_resample(scene.sec, sec, az, az)
+    assert np.array_equal(np.abs(got) > 0, np.abs(want) > 0)
+    assert rel_err(got, want) < 2e-5
+
+
 @pytest.mark.parametrize("cols", [317, 318])
 def test_resample_plain_load_path(cuda, scene, cols):
     """Widths whose offset rows are not a multiple of 16 bytes (no tensor map)
