@@ -4,18 +4,33 @@
 // cuFFT forward, gaussian_filter, patchwise_normalize, spectrum_enhancement,
 // cuFFT inverse, batched_overlap_add, normalize_output), reference
 // csrc/src/goldstein.cu:87-408, with two kernels:
-//   1. goldstein_patch_kernel -- one warp per 32x32 patch: coalesced patch
-//      load into shared memory, 2-D FFT as 32-point radix-2 FFTs held in
-//      registers (rows, then columns through a padded shared tile), |F|,
-//      7x7 circular smoothing, patch-mean normalisation, S^alpha weighting,
-//      inverse 2-D FFT, triangular weight and 1/n^2 scale; the weighted patch
-//      is written to scratch.
-//   2. goldstein_gather_kernel -- one thread per output pixel sums the (up to
-//      16) weighted patches covering it in a fixed order and divides by the
-//      summed weights.  No atomics: the result is deterministic.
+//   1. goldstein_run_kernel -- one warp per run of 1 to 8 vertically
+//      neighbouring 32x32 patches.  Per patch: coalesced load, 2-D FFT as
+//      32-point radix-2 FFTs held in registers (columns, then rows through a
+//      padded shared tile), |F|, 7x7 circular smoothing, patch-mean
+//      normalisation, S^alpha weighting, inverse 2-D FFT, triangular weight
+//      and 1/n^2 scale; rows add up over the run in shared memory and leave
+//      for the scratch once no later patch of the run reaches them.
+//   2. goldstein_gather_kernel -- each output pixel sums the runs covering it
+//      (4 columns by 1 or 2 runs where runs are long) in a fixed order and
+//      divides by the summed weights.  No atomics: the result is
+//      deterministic.
+//
+// 3217 x 1391 samples (68 400 patches): 318 us in kernel 1 and 62 us in kernel
+// 2, against 405 and 184 with single patches as the unit.  Kernel 1 is bound
+// by instruction issue and the FP32 pipe together (3000 instructions a patch,
+// 58 % of the issue slots, packed FP32 instructions for two slots of the pipe
+// each), kernel 2 by the latency of its loads from L2 and memory.  Against the
+// former unit: the runs cut the scratch traffic from 8 KB a patch each way to
+// 2.8 KB; columns first, so that loads, sums and stores are coalesced without a
+// transpose (two per patch, not four); one copy of the FFT's code for the four
+// transforms (unrolled four times, a fifth of the issue slots waited for the
+// instruction cache); multiplications folded into the butterflies' additions;
+// the patch mean from |F|, so that smoothed values are not kept.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "s1b.h"
@@ -28,99 +43,91 @@ namespace {
 
 constexpr int GN = 32;        // patch size (s1proc filter.window_size)
 constexpr int GSTEP = GN / 4; // patch step, goldstein.cu:334
-constexpr int GWARPS = 4;     // patches per CTA
-// CTAs per SM the patch kernels are compiled for: 128 registers per thread,
-// the FFT's 32 complex values in registers with a small spill (measured
-// 1.14 ms per 27-pair frame against 1.41 ms at 168 registers and 3 CTAs/SM)
-constexpr int GCTAS_PER_SM = 4;
+// One warp per CTA, so that the run's addresses are uniform: 394 us per
+// 3217 x 1391 image against 405 with two.  12 CTAs per SM: 168 registers (the
+// 32 complex values of a transform and the 32 magnitudes) and 17 KB of shared
+// memory each.
+constexpr int GCTAS_PER_SM = 12;
+// Patches of the longest run, and how many runs an image has at least before
+// its runs are made longer: a wave of one-warp CTAs.  Longer runs save scratch
+// traffic, but a patch of a run waits for the one before it: 1217 x 391 samples
+// (6850 patches) take 53 us in runs of 2 and 68 in runs of 8; 3217 x 1391 394
+// in runs of 8 and 418 in runs of 16.
+constexpr int GRUN_MAX = 8;
+constexpr int GRUN_JOBS = 148 * GCTAS_PER_SM;
+// Gathering: columns of a CTA, and output pixels from which a thread takes
+// eight rows (columns and weights found once) instead of one (more loads in
+// flight): 387 us against 394 at 3217 x 1391, 59 against 53 at 1217 x 391, 46
+// against 33 at 430 x 470.
+constexpr int GGATHER = 256;
+constexpr int64_t kGatherRows8 = 1 << 20;
 
-// exp(2 pi i k / 32), k = 0..15, from cos/sin of 2 pi k / 32 evaluated in
-// 50-digit decimal arithmetic.
-__constant__ float2 c_tw[16] = {
-    {1.0f, 0.0f},
-    {0.9807852804032304f, 0.19509032201612828f},
-    {0.9238795325112867f, 0.3826834323650898f},
-    {0.8314696123025452f, 0.5555702330196022f},
-    {0.7071067811865476f, 0.7071067811865476f},
-    {0.5555702330196022f, 0.8314696123025452f},
-    {0.3826834323650898f, 0.9238795325112867f},
-    {0.19509032201612828f, 0.9807852804032304f},
-    {0.0f, 1.0f},
-    {-0.19509032201612828f, 0.9807852804032304f},
-    {-0.3826834323650898f, 0.9238795325112867f},
-    {-0.5555702330196022f, 0.8314696123025452f},
-    {-0.7071067811865476f, 0.7071067811865476f},
-    {-0.8314696123025452f, 0.5555702330196022f},
-    {-0.9238795325112867f, 0.3826834323650898f},
-    {-0.9807852804032304f, 0.19509032201612828f},
-};
+// cos(pi k / 16) and tan(pi k / 16), k = 0..4, evaluated in 50-digit decimal
+// arithmetic: a rotation exp(-pi i k / 16) is taken as the larger of its
+// cosine and sine times a shear by the tangent or cotangent (at most 1).
+constexpr float kCos[5] = {1.0f, 0.9807852804032304f, 0.9238795325112867f, 0.8314696123025452f, 0.7071067811865476f};
+constexpr float kTan[5] = {0.0f, 0.1989123673796580f, 0.4142135623730950f, 0.6681786379192989f, 1.0f};
 
-// The reference project's 7x7 smoothing table, goldstein.cu:43-52 (row
-// ky = -3..3, column kx = -3..3).  Kept as given: the filter output depends
-// on these exact values.
-__constant__ float c_gauss[49] = {
-    0.000004f, 0.000088f, 0.000543f, 0.000948f, 0.000543f, 0.000088f, 0.000004f,
-    0.000088f, 0.001915f, 0.011776f, 0.020584f, 0.011776f, 0.001915f, 0.000088f,
-    0.000543f, 0.011776f, 0.072410f, 0.126584f, 0.072410f, 0.011776f, 0.000543f,
-    0.000948f, 0.020584f, 0.126584f, 0.221141f, 0.126584f, 0.020584f, 0.000948f,
-    0.000543f, 0.011776f, 0.072410f, 0.126584f, 0.072410f, 0.011776f, 0.000543f,
-    0.000088f, 0.001915f, 0.011776f, 0.020584f, 0.011776f, 0.001915f, 0.000088f,
-    0.000004f, 0.000088f, 0.000543f, 0.000948f, 0.000543f, 0.000088f, 0.000004f};
+// The reference project's 7x7 smoothing table, goldstein.cu:43-52: even in both
+// offsets and symmetric, so the entries g[a][b], a, b = 0..3, in pairs (g[a][0],
+// g[a][1]), (g[a][2], g[a][3]).  Kept as given: the filter output depends on
+// these exact values.
+__constant__ float2 c_gauss2[8] = {{0.221141f, 0.126584f}, {0.020584f, 0.000948f}, {0.126584f, 0.072410f},
+                                   {0.011776f, 0.000543f}, {0.020584f, 0.011776f}, {0.001915f, 0.000088f},
+                                   {0.000948f, 0.000543f}, {0.000088f, 0.000004f}};
+// Sum of the table: g[0][0] + 4 sum_a g[a][0] + 4 sum_ab g[a][b], a, b = 1..3.
+constexpr float kGaussSum =
+    (float)(0.221141 + 4 * (0.126584 + 0.020584 + 0.000948) +
+            4 * (0.072410 + 0.001915 + 0.000004 + 2 * (0.011776 + 0.000543 + 0.000088)));
 
 __host__ __device__ constexpr int brev5(int i) {
   return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
 }
 
-// One radix-2 stage (butterfly span m = 2^S) of the 32-point FFT; a template
-// per stage so that every index is a compile-time constant and x stays in
-// registers.  The twiddles 1 and -+i are applied as copies and swaps: the
-// same values the multiplication gives for finite samples, without its
-// multiplies (46 of the 80 butterflies of a transform).
-template <int S, bool kInverse>
-__device__ __forceinline__ void fft32_stage(float2 (&x)[GN]) {
-  constexpr int m = 1 << S, half = m >> 1, stride = GN / m;
-#pragma unroll
-  for (int k = 0; k < GN; k += m) {
-#pragma unroll
-    for (int j = 0; j < half; ++j) {
-      const int tw = j * stride;
-      const float2 b = x[k + j + half];
-      float2 t;
-      if (tw == 0) {
-        t = b;
-      } else if (tw == GN / 4) {  // exp(-+i pi / 2)
-        t = kInverse ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x);
-      } else {
-        float2 w = c_tw[tw];
-        if (!kInverse) w.y = -w.y;
-        t = make_float2(w.x * b.x - w.y * b.y, w.x * b.y + w.y * b.x);
-      }
-      const float2 u = x[k + j];
-      x[k + j] = make_float2(u.x + t.x, u.y + t.y);
-      x[k + j + half] = make_float2(u.x - t.x, u.y - t.y);
-    }
+// Radix-2 butterfly with the twiddle exp(-2 pi i k / 32): u + w b into u, u -
+// w b into b.  w b = c (shear of b), so the multiply by c rides on the two
+// additions: two FFMA and two FFMA2, against two FMUL, an FFMA2 and two
+// additions for the product formed first.
+template <int k>
+__device__ __forceinline__ void butterfly(float2 &u, float2 &b) {
+  const float2 a = u;
+  if constexpr (k == 0) {
+    u = __fadd2_rn(a, b);
+    b = __ffma2_rn(make_float2(-1.f, -1.f), b, a);
+  } else if constexpr (k == 8) {  // -i b
+    u = make_float2(a.x + b.y, a.y - b.x);
+    b = make_float2(a.x - b.y, a.y + b.x);
+  } else {
+    // exp(-i t) b = cos t (b.x + tan t b.y, b.y - tan t b.x)
+    //             = sin t (b.y + cot t b.x, -b.x + cot t b.y)
+    constexpr int m = k < 8 ? k : 16 - k;  // mirrored at pi / 2
+    constexpr bool by_cos = m <= 4;
+    constexpr float tn = k < 8 ? kTan[by_cos ? m : 8 - m] : -kTan[by_cos ? m : 8 - m];
+    constexpr float c = by_cos ? (k < 8 ? kCos[m] : -kCos[m]) : kCos[8 - m];
+    const float2 t = by_cos ? make_float2(fmaf(tn, b.y, b.x), fmaf(-tn, b.x, b.y))
+                            : make_float2(fmaf(tn, b.x, b.y), fmaf(tn, b.y, -b.x));
+    u = __ffma2_rn(make_float2(c, c), t, a);
+    b = __ffma2_rn(make_float2(-c, -c), t, a);
   }
 }
 
-// In-place 32-point DFT of x (natural order in and out), radix-2
-// decimation in time.  Forward: exp(-2 pi i jk/32); inverse: exp(+...),
-// unnormalised (cuFFT's convention).
-template <bool kInverse>
-__device__ __forceinline__ void fft32(float2 (&x)[GN]) {
+template <int S, int J>
+__device__ __forceinline__ void fft32_twiddle(float2 (&x)[GN]) {
+  constexpr int m = 1 << S, half = m >> 1;
 #pragma unroll
-  for (int i = 0; i < GN; ++i) {
-    const int j = brev5(i);
-    if (j > i) {
-      const float2 t = x[i];
-      x[i] = x[j];
-      x[j] = t;
-    }
-  }
-  fft32_stage<1, kInverse>(x);
-  fft32_stage<2, kInverse>(x);
-  fft32_stage<3, kInverse>(x);
-  fft32_stage<4, kInverse>(x);
-  fft32_stage<5, kInverse>(x);
+  for (int k = 0; k < GN; k += m) butterfly<J * (GN / m)>(x[k + J], x[k + J + half]);
+  if constexpr (J + 1 < half) fft32_twiddle<S, J + 1>(x);
+}
+
+// 32-point forward DFT, exp(-2 pi i jk / 32), unnormalised: radix-2
+// decimation in time, x[brev5(j)] = element j on entry, natural order on
+// return.
+__device__ __forceinline__ void fft32(float2 (&x)[GN]) {
+  fft32_twiddle<1, 0>(x);
+  fft32_twiddle<2, 0>(x);
+  fft32_twiddle<3, 0>(x);
+  fft32_twiddle<4, 0>(x);
+  fft32_twiddle<5, 0>(x);
 }
 
 __device__ __forceinline__ float tri_weight(int t) {  // goldstein.cu:257-258
@@ -132,163 +139,6 @@ __device__ __forceinline__ int patch_origin(int p, int n) {  // goldstein.cu:308
   return o + GN > n ? n - GN : o;
 }
 
-// Patch p of an nrow x ncol image, by one warp with its padded 32x33 tile
-// T; |F| reuses the tile once the column FFT inputs are in registers.
-__device__ __forceinline__ void goldstein_patch(const float2 *__restrict__ in, float2 *__restrict__ patches,
-                                                int nrow, int ncol, int n_win_j, float alpha, int p,
-                                                float2 (*T)[GN + 1]) {
-  const int lane = threadIdx.x & 31;
-  const int i1 = patch_origin(p / n_win_j, nrow);
-  const int j1 = patch_origin(p % n_win_j, ncol);
-  float(*M)[GN + 1] = reinterpret_cast<float(*)[GN + 1]>(&T[0][0]);
-  float2 x[GN];
-  // all 32 row loads in flight at once (one L2 round trip per patch), then
-  // the transpose through the tile
-#pragma unroll
-  for (int r = 0; r < GN; ++r) x[r] = __ldg(in + (size_t)(i1 + r) * ncol + j1 + lane);
-#pragma unroll
-  for (int r = 0; r < GN; ++r) T[r][lane] = x[r];
-  __syncwarp();
-  // forward FFT along rows (lane = row)
-#pragma unroll
-  for (int c = 0; c < GN; ++c) x[c] = T[lane][c];
-  fft32<false>(x);
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < GN; ++c) T[lane][c] = x[c];
-  __syncwarp();
-  // forward FFT along columns (lane = column kx); x[ky] = F[ky][kx]
-#pragma unroll
-  for (int r = 0; r < GN; ++r) x[r] = T[r][lane];
-  fft32<false>(x);
-  __syncwarp();
-#pragma unroll
-  // |F|: spectral magnitudes of a 32 x 32 patch of interferogram samples are
-  // far from float overflow, so the plain root of the squared sum serves
-  for (int r = 0; r < GN; ++r) M[r][lane] = sqrtf(fmaf(x[r].x, x[r].x, x[r].y * x[r].y));
-  __syncwarp();
-  // 7x7 circular smoothing of |F| (goldstein.cu:105-119) and its patch sum.
-  // The table is even in both offsets, g[ky][kx] = g[|ky|][|kx|], so
-  //   S[y][x] = W0[y][x] + sum_{b=1..3} (Wb[y][x - b] + Wb[y][x + b]),
-  //   Wb[y][x] = sum_{a=0..3} g[a][b] (M[y - a][x] + M[y + a][x])  (a = 0 once):
-  // the four vertical filters Wb run down the lane's own column from a
-  // sliding window of seven rows, the horizontal offsets are lane shuffles
-  // (their wrap-around is the circular boundary).
-  float S[GN];
-  float psum = 0.f;
-  {
-    float win[7];  // M[y - 3 .. y + 3][lane]
-#pragma unroll
-    for (int k = 0; k < 6; ++k) win[k + 1] = M[(k - 3 + GN) & (GN - 1)][lane];
-#pragma unroll
-    for (int y = 0; y < GN; ++y) {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) win[k] = win[k + 1];
-      win[6] = M[(y + 3) & (GN - 1)][lane];
-      const float p1 = win[2] + win[4], p2 = win[1] + win[5], p3 = win[0] + win[6];
-      float w[4];
-#pragma unroll
-      for (int b = 0; b < 4; ++b)  // g[a][b] = c_gauss[(3 - a) * 7 + 3 + b]
-        w[b] = fmaf(c_gauss[21 + 3 + b], win[3],
-                    fmaf(c_gauss[14 + 3 + b], p1, fmaf(c_gauss[7 + 3 + b], p2, c_gauss[3 + b] * p3)));
-      float s = w[0];
-#pragma unroll
-      for (int b = 1; b < 4; ++b)
-        s += __shfl_sync(0xffffffffu, w[b], (lane - b) & (GN - 1)) + __shfl_sync(0xffffffffu, w[b], (lane + b) & (GN - 1));
-      S[y] = s;
-      psum += s;
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, off);
-  // patch-mean normalisation and S^alpha weighting (goldstein.cu:125-176)
-  const float mean = psum / (float)(GN * GN);
-  const bool ok = mean > 1e-8f;
-  const float inv = 1.0f / mean;
-#pragma unroll
-  for (int y = 0; y < GN; ++y) {
-    // S^alpha through the hardware exp2/log2 (relative error ~1e-6, far
-    // below the filter's float tolerance); 0^alpha = 0 for alpha > 0, and a
-    // NaN weight (0^0) leaves F unscaled, as a weight of 1 would
-    const float w = __powf(ok ? S[y] * inv : 0.0f, alpha);
-    if (w > 0.0f) {
-      x[y].x *= w;
-      x[y].y *= w;
-    }
-  }
-  // inverse FFT along columns, then rows
-  fft32<true>(x);
-  __syncwarp();
-#pragma unroll
-  for (int y = 0; y < GN; ++y) T[y][lane] = x[y];
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < GN; ++c) x[c] = T[lane][c];
-  fft32<true>(x);
-  // triangular weight and 1/n^2 (goldstein.cu:257-269); stage for a
-  // coalesced store
-  const float wy = tri_weight(lane);
-  const float norm = 1.0f / (float)(GN * GN);
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < GN; ++c) {
-    const float w = (tri_weight(c) + wy) * norm;
-    T[lane][c] = make_float2(x[c].x * w, x[c].y * w);
-  }
-  __syncwarp();
-  float2 *dst = patches + (size_t)p * (GN * GN);
-#pragma unroll 8
-  for (int r = 0; r < GN; ++r) __stcg(dst + r * GN + lane, T[r][lane]);
-}
-
-__global__ __launch_bounds__(32 * GWARPS, GCTAS_PER_SM) void goldstein_patch_kernel(
-    const float2 *__restrict__ in, float2 *__restrict__ patches, int nrow, int ncol, int n_win_i,
-    int n_win_j, float alpha) {
-  __shared__ float2 sT[GWARPS][GN][GN + 1];
-  const int warp = threadIdx.x >> 5;
-  const int p = blockIdx.x * GWARPS + warp;
-  if (p >= n_win_i * n_win_j) return;  // warp-uniform; only __syncwarp below
-  goldstein_patch(in, patches, nrow, ncol, n_win_j, alpha, p, sT[warp]);
-}
-
-// Output pixel (y, x): fixed-order overlap-add of its covering patches.
-__device__ __forceinline__ void goldstein_gather(const float2 *__restrict__ patches, float2 *__restrict__ out,
-                                                 int nrow, int ncol, int n_win_i, int n_win_j, int y, int x) {
-  float ax = 0.f, ay = 0.f, wsum = 0.f;
-  const int pi0 = y >= GN - 1 ? (y - (GN - 1) + GSTEP - 1) / GSTEP : 0;
-  const int pj0 = x >= GN - 1 ? (x - (GN - 1) + GSTEP - 1) / GSTEP : 0;
-  for (int pi = pi0; pi < n_win_i; ++pi) {
-    const int i1 = patch_origin(pi, nrow);
-    if (i1 > y) break;
-    if (y >= i1 + GN) continue;
-    const int ty = y - i1;
-    const float wy = tri_weight(ty);
-    for (int pj = pj0; pj < n_win_j; ++pj) {
-      const int j1 = patch_origin(pj, ncol);
-      if (j1 > x) break;
-      if (x >= j1 + GN) continue;
-      const int tx = x - j1;
-      const float2 v = __ldcg(patches + ((size_t)pi * n_win_j + pj) * (GN * GN) + ty * GN + tx);
-      ax += v.x;
-      ay += v.y;
-      wsum += tri_weight(tx) + wy;
-    }
-  }
-  if (wsum > 0.f) {  // goldstein.cu:287-291
-    ax /= wsum;
-    ay /= wsum;
-  }
-  out[(size_t)y * ncol + x] = make_float2(ax, ay);
-}
-
-__global__ __launch_bounds__(256) void goldstein_gather_kernel(const float2 *__restrict__ patches,
-                                                               float2 *__restrict__ out, int nrow,
-                                                               int ncol, int n_win_i, int n_win_j) {
-  const int x = blockIdx.y * 256 + threadIdx.x;
-  if (x >= ncol) return;
-  goldstein_gather(patches, out, nrow, ncol, n_win_i, n_win_j, blockIdx.x, x);
-}
-
 __host__ __device__ inline void patch_grid(int nrow, int ncol, int &n_win_i, int &n_win_j) {  // goldstein.cu:335-340
   n_win_i = (int)ceilf((float)nrow / GSTEP) - 3;
   n_win_j = (int)ceilf((float)ncol / GSTEP) - 3;
@@ -296,38 +146,286 @@ __host__ __device__ inline void patch_grid(int nrow, int ncol, int &n_win_i, int
   if (n_win_j <= 0) n_win_j = 1;
 }
 
+// Patch rows that one warp takes in a run, for an image of ni x nj patches: a
+// pure function of the image, so that a filter of many images sums in the
+// order of the single one.
+__host__ __device__ inline int run_patches(int ni, int nj) {
+  int k = 1;
+  while (k < GRUN_MAX && 2 * k <= ni && (int64_t)ni * nj >= (int64_t)(2 * k) * GRUN_JOBS) k *= 2;
+  return k;
+}
+
+// Scratch rows of a run of k patches (32 columns each).  Runs x rows never
+// exceed ni x 32: ceil(ni / k) (k + 3) / 4 <= ni for k <= ni.
+__host__ __device__ inline int run_rows(int k) { return GSTEP * (k - 1) + GN; }
+
+// Magnitude within one unit in the last place: the square root of the sum of
+// squares, which is far from float overflow for interferogram samples.
+__device__ __forceinline__ float magnitude(float2 v) {
+  float m;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(m) : "f"(fmaf(v.x, v.x, v.y * v.y)));
+  return m;
+}
+
+// The spectrum's weights, by the warp that holds it (lane = ky, x[kx]): F
+// times S^alpha, S the smoothed |F| over its patch mean (goldstein.cu:105-176).
+// Returns the conjugates in the order that fft32 reads, x[brev5(kx)].
+__device__ __forceinline__ void goldstein_weigh(float2 (&x)[GN], float alpha) {
+  const int lane = threadIdx.x & 31;
+  float m[GN];
+  float psum = 0.f;
+#pragma unroll
+  for (int c = 0; c < GN; ++c) {
+    m[c] = magnitude(x[c]);
+    psum += m[c];
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, off);
+  // the smoothing is circular, so the mean of S is that of |F| times the sum
+  // of the table
+  const float mean = psum * (kGaussSum / (float)(GN * GN));
+  const float inv = mean > 1e-8f ? 1.0f / mean : 0.0f;
+  // 7x7 circular smoothing.  The table is even in both offsets and symmetric:
+  //   S[kx] = W0[kx] + sum_{b=1..3} (Wb of the lanes ky - b and ky + b),
+  //   Wb[kx] = sum_{a=0..3} g[a][b] (M[kx - a] + M[kx + a])  (a = 0 once):
+  // the four filters Wb run along the lane's own spectrum, two at a time from
+  // a sliding window of seven magnitudes, each kept twice; the offsets in ky
+  // are lane shuffles (their wrap-around is the circular boundary).
+  float2 win[7];
+  float first[3];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) win[i + 1] = make_float2(m[(i + GN - 3) & (GN - 1)], m[(i + GN - 3) & (GN - 1)]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) first[i] = m[i];
+#pragma unroll
+  for (int c = 0; c < GN; ++c) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) win[i] = win[i + 1];
+    const float last = c + 3 < GN ? m[(c + 3) & (GN - 1)] : first[(c + 3) & (GN - 1) & 3];
+    win[6] = make_float2(last, last);
+    const float2 p1 = __fadd2_rn(win[2], win[4]), p2 = __fadd2_rn(win[1], win[5]), p3 = __fadd2_rn(win[0], win[6]);
+    const float2 w01 = __ffma2_rn(c_gauss2[0], win[3], __ffma2_rn(c_gauss2[2], p1, __ffma2_rn(c_gauss2[4], p2, __fmul2_rn(c_gauss2[6], p3))));
+    const float2 w23 = __ffma2_rn(c_gauss2[1], win[3], __ffma2_rn(c_gauss2[3], p1, __ffma2_rn(c_gauss2[5], p2, __fmul2_rn(c_gauss2[7], p3))));
+    float s = w01.x;
+    s += __shfl_sync(0xffffffffu, w01.y, (lane - 1) & (GN - 1)) + __shfl_sync(0xffffffffu, w01.y, (lane + 1) & (GN - 1));
+    s += __shfl_sync(0xffffffffu, w23.x, (lane - 2) & (GN - 1)) + __shfl_sync(0xffffffffu, w23.x, (lane + 2) & (GN - 1));
+    s += __shfl_sync(0xffffffffu, w23.y, (lane - 3) & (GN - 1)) + __shfl_sync(0xffffffffu, w23.y, (lane + 3) & (GN - 1));
+    // S^alpha through the hardware exp2/log2 (relative error ~1e-6, far below
+    // the filter's float tolerance); 0^alpha = 0 for alpha > 0, and a NaN
+    // weight (0^0) leaves F unscaled, as a weight of 1 would
+    float e;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(s * inv));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(alpha * e));
+    m[c] = e > 0.0f ? e : 1.0f;
+  }
+#pragma unroll
+  for (int c = 0; c < GN; ++c) {
+    const int d = brev5(c);
+    if (d < c) continue;
+    const float2 t = __fmul2_rn(x[c], make_float2(m[c], -m[c]));
+    if (d > c) x[c] = __fmul2_rn(x[d], make_float2(m[d], -m[d]));
+    x[d] = t;
+  }
+}
+
+struct GoldsteinTile {
+  float2 T[GN][GN + 1];  // transposes
+  float2 sums[GN][GN];   // of the rows that the next patch reaches too
+};
+
+// Run `job` (runs in row-major order over (run, patch column)) of an nrow x
+// ncol image, by one warp.
+__device__ __forceinline__ void goldstein_run(const float2 *__restrict__ in, float2 *__restrict__ runs, int nrow,
+                                              int ncol, int ni, int nj, float alpha, int job, GoldsteinTile &tile) {
+  float2(*T)[GN + 1] = tile.T;
+  const int lane = threadIdx.x & 31;
+  const int k = run_patches(ni, nj);
+  const int p0 = job / nj * k, p1 = min(ni, p0 + k);
+  const int j1 = patch_origin(job % nj, ncol);
+  float2 *dst = runs + (size_t)job * run_rows(k) * GN + lane;
+  const float wx = tri_weight(lane);
+  // weighted sums so far of rows i1 .. i1 + 31 at column j1 + lane; the lane's
+  // own, and the rows of i1 + 24 on stay zero (a patch keeps 32 - step < 32 - 7
+  // rows, or fewer zeros above them after the shorter last step)
+  float2 *sums = &tile.sums[0][lane];
+#pragma unroll
+  for (int r = 0; r < GN; ++r) sums[r * GN] = make_float2(0.f, 0.f);
+  int i1 = patch_origin(p0, nrow);
+#pragma unroll 1
+  for (int p = p0; p < p1; ++p) {
+    float2 x[GN];
+    const float2 *src = in + (size_t)i1 * ncol + j1 + lane;
+#pragma unroll
+    for (int r = 0; r < GN; ++r) x[brev5(r)] = __ldg(src + (size_t)r * ncol);
+    // forward transform along the lane's column, then, transposed, along the
+    // lane's row; the inverse the same way from conjugate to conjugate.  One
+    // copy of the transform's code serves the four.
+#pragma unroll 1
+    for (int pass = 0; pass < 4; ++pass) {
+      fft32(x);
+      if (!(pass & 1)) {
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < GN; ++r) T[r][lane] = x[r];
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < GN; ++c) x[brev5(c)] = T[lane][c];
+      } else if (pass == 1) {
+        goldstein_weigh(x, alpha);
+      }
+    }
+    // triangular weight and 1/n^2 (goldstein.cu:257-269); rows that the next
+    // patch of the run does not reach are complete
+    const int next = p + 1 < p1 ? patch_origin(p + 1, nrow) : i1 + GN;
+    const int step = next - i1;
+    float2 *keep = sums - step * GN;
+#pragma unroll
+    for (int r = 0; r < GN; ++r) {
+      const float w = (wx + tri_weight(r)) * (1.0f / (float)(GN * GN));
+      const float2 v = __ffma2_rn(x[r], make_float2(w, -w), sums[r * GN]);
+      if (r < step)
+        __stcg(dst + r * GN, v);
+      else
+        keep[r * GN] = v;
+    }
+    dst += step * GN;
+    i1 = next;
+  }
+}
+
+__global__ __launch_bounds__(32, GCTAS_PER_SM) void goldstein_run_kernel(
+    const float2 *__restrict__ in, float2 *__restrict__ runs, int nrow, int ncol, int ni, int nj, float alpha) {
+  __shared__ GoldsteinTile tile;
+  goldstein_run(in, runs, nrow, ncol, ni, nj, alpha, blockIdx.x, tile);
+}
+
+// Output rows y0 .. y0 + R - 1 of column x, within a multiple of 8 and the
+// next: each pixel the sum of the runs that
+// cover it (run by run, columns ascending) over its weights.  The weights wx +
+// wy of the covering patches are whole numbers: their sum over the ny x nx of
+// them is exact as ny sum(wx) + nx sum(wy).
+template <int R>
+__device__ __forceinline__ void goldstein_gather(const float2 *__restrict__ runs, float2 *__restrict__ out, int nrow,
+                                                 int ncol, int ni, int nj, int y0, int x) {
+  const int k = run_patches(ni, nj), rows = run_rows(k);
+  const int g = y0 / GSTEP, ny0 = min(R, nrow - y0);
+  // the patch columns pj0 .. pj0 + 3 that lie before the last one, and the last
+  const int pj0 = max(0, (x - (GN - 1) + GSTEP - 1) / GSTEP);
+  bool cov[5];
+  size_t off[5];  // of column x in the area of each
+  float wx = 0.f, nx = 0.f;
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const int pj = j < 4 ? pj0 + j : nj - 1, tx = x - (j < 4 ? pj * GSTEP : patch_origin(pj, ncol));
+    cov[j] = (j == 4 || pj < nj - 1) && tx >= 0;
+    off[j] = (size_t)pj * (rows * GN) + tx;
+    wx += cov[j] ? tri_weight(tx) : 0.f;
+    nx += cov[j] ? 1.f : 0.f;
+  }
+  float2 acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+  const int first = max(0, g - 3), last = patch_origin(ni - 1, nrow) < y0 + ny0 ? ni - 1 : g;
+  for (int run = first / k; run <= last / k; ++run) {
+    const int o = patch_origin(run * k, nrow), end = patch_origin(min(ni, run * k + k) - 1, nrow) + GN;
+    const float2 *src = runs + (size_t)run * nj * rows * GN + (y0 - o) * GN;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r < ny0 && y0 + r >= o && y0 + r < end) {
+        float2 v[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) v[j] = cov[j] ? __ldcg(src + r * GN + off[j]) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) acc[r] = __fadd2_rn(acc[r], v[j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (r >= ny0) break;
+    float wy = 0.f, ny = 0.f;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int pi = i < 4 ? first + i : ni - 1, ty = y0 + r - (i < 4 ? pi * GSTEP : patch_origin(pi, nrow));
+      if ((i == 4 || pi < ni - 1) && ty >= 0 && ty < GN) {
+        wy += tri_weight(ty);
+        ny += 1.f;
+      }
+    }
+    const float wsum = ny * wx + nx * wy;
+    if (wsum > 0.f) {  // goldstein.cu:287-291
+      acc[r].x /= wsum;
+      acc[r].y /= wsum;
+    }
+    out[(size_t)(y0 + r) * ncol + x] = acc[r];
+  }
+}
+
+template <int R>
+__global__ __launch_bounds__(GGATHER) void goldstein_gather_kernel(const float2 *__restrict__ runs,
+                                                                   float2 *__restrict__ out, int nrow, int ncol,
+                                                                   int ni, int nj) {
+  const int x = blockIdx.y * GGATHER + threadIdx.x;
+  if (x >= ncol) return;
+  goldstein_gather<R>(runs, out, nrow, ncol, ni, nj, blockIdx.x * R, x);
+}
+
+__host__ __device__ inline int run_jobs(int ni, int nj) {
+  const int k = run_patches(ni, nj);
+  return (ni + k - 1) / k * nj;
+}
+
+
 
 // ------------------------------------------------------------ frame stages
 // Goldstein of every pair's interferogram: blockIdx.y = pair.  Pairs too
 // small to filter get filt = ifg from the gather kernel.
-__global__ __launch_bounds__(32 * GWARPS, GCTAS_PER_SM) void frame_goldstein_patch_kernel(const FrameDev d, const FrameIO io) {
-  __shared__ float2 sT[GWARPS][GN][GN + 1];
+__global__ __launch_bounds__(32, GCTAS_PER_SM) void frame_goldstein_run_kernel(const FrameDev d, const FrameIO io) {
+  __shared__ GoldsteinTile tile;
   const int k = blockIdx.y;
   const s1b_frame_pair_t &r = io.pout[k];
   if (!r.ok || !r.filtered) return;
   int ni, nj;
   patch_grid(r.nrow_ml, r.ncol_ml, ni, nj);
-  const int warp = threadIdx.x >> 5;
-  const int p = blockIdx.x * GWARPS + warp;
-  if (p >= ni * nj) return;  // warp-uniform
+  if ((int)blockIdx.x >= run_jobs(ni, nj)) return;
   const FramePair &pr = d.pairs[k];
-  goldstein_patch(io.ifg + pr.ml_off, io.work + pr.scratch_off, r.nrow_ml, r.ncol_ml, nj, d.alpha, p, sT[warp]);
+  goldstein_run(io.ifg + pr.ml_off, io.work + pr.scratch_off, r.nrow_ml, r.ncol_ml, ni, nj, d.alpha, blockIdx.x,
+                tile);
 }
 
-__global__ __launch_bounds__(256) void frame_goldstein_gather_kernel(const FrameDev d, const FrameIO io) {
+template <int R>
+__global__ __launch_bounds__(GGATHER) void frame_goldstein_gather_kernel(const FrameDev d, const FrameIO io) {
   const int k = blockIdx.z;
   const s1b_frame_pair_t &r = io.pout[k];
-  const int y = blockIdx.x, x = blockIdx.y * 256 + threadIdx.x;
-  if (!r.ok || y >= r.nrow_ml || x >= r.ncol_ml) return;
+  const int y0 = blockIdx.x * R, x = blockIdx.y * GGATHER + threadIdx.x;
+  if (!r.ok || y0 >= r.nrow_ml || x >= r.ncol_ml) return;
   const FramePair &pr = d.pairs[k];
   if (r.filtered) {
     int ni, nj;
     patch_grid(r.nrow_ml, r.ncol_ml, ni, nj);
-    goldstein_gather(io.work + pr.scratch_off, io.filt + pr.ml_off, r.nrow_ml, r.ncol_ml, ni, nj, y, x);
+    goldstein_gather<R>(io.work + pr.scratch_off, io.filt + pr.ml_off, r.nrow_ml, r.ncol_ml, ni, nj, y0, x);
   } else {
-    const size_t o = pr.ml_off + (size_t)y * r.ncol_ml + x;
-    io.filt[o] = io.ifg[o];
+    for (int y = y0; y < min(y0 + R, r.nrow_ml); ++y) {
+      const size_t o = pr.ml_off + (size_t)y * r.ncol_ml + x;
+      io.filt[o] = io.ifg[o];
+    }
   }
+}
+
+int launch_goldstein(const void *in, void *out, int nrow, int ncol, int ni, int nj, float alpha, void *scratch,
+                     cudaStream_t st) {
+  goldstein_run_kernel<<<run_jobs(ni, nj), 32, 0, st>>>((const float2 *)in, (float2 *)scratch, nrow, ncol, ni, nj,
+                                                        alpha);
+  const int s = s1b_launch_status();
+  if (s) return s;
+  const dim3 grid(nrow, (ncol - 1) / GGATHER + 1);
+  if ((int64_t)nrow * ncol >= kGatherRows8) {
+    goldstein_gather_kernel<GSTEP><<<dim3((nrow - 1) / GSTEP + 1, grid.y), GGATHER, 0, st>>>(
+        (const float2 *)scratch, (float2 *)out, nrow, ncol, ni, nj);
+  } else {
+    goldstein_gather_kernel<1><<<grid, GGATHER, 0, st>>>((const float2 *)scratch, (float2 *)out, nrow, ncol, ni, nj);
+  }
+  return s1b_launch_status();
 }
 
 }  // namespace
@@ -350,18 +448,9 @@ extern "C" int s1b_goldstein(const void *in, void *out, int32_t nrow, int32_t nc
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_goldstein: scratch buffer too small");
   int ni, nj;
   patch_grid(nrow, ncol, ni, nj);
-  const int64_t npatch = (int64_t)ni * nj;
-  if ((npatch + GWARPS - 1) / GWARPS > 0x7fffffff || (ncol + 255) / 256 > 65535)
+  if ((int64_t)ni * nj > 0x7fffffff || (ncol + 255) / 256 > 65535)
     return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_goldstein: image too large");
-  cudaStream_t st = (cudaStream_t)stream;
-  goldstein_patch_kernel<<<(unsigned)((npatch + GWARPS - 1) / GWARPS), 32 * GWARPS, 0, st>>>(
-      (const float2 *)in, (float2 *)scratch, nrow, ncol, ni, nj, alpha);
-  int s = s1b_launch_status();
-  if (s) return s;
-  dim3 grid(nrow, (ncol + 255) / 256);
-  goldstein_gather_kernel<<<grid, 256, 0, st>>>((const float2 *)scratch, (float2 *)out, nrow, ncol,
-                                                ni, nj);
-  return s1b_launch_status();
+  return launch_goldstein(in, out, nrow, ncol, ni, nj, alpha, scratch, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -461,16 +550,9 @@ extern "C" int s1b_goldstein_noalloc(const void *in, void *out, int32_t nrow, in
   void *scratch = nullptr;
   int s = noalloc_scratch(&scratch);
   if (s) return s;
-  // every patch slot used below is written by the patch kernel before the
-  // gather reads it, so nothing left by an earlier call needs clearing
-  cudaStream_t st = (cudaStream_t)stream;
-  goldstein_patch_kernel<<<(unsigned)((npatch + GWARPS - 1) / GWARPS), 32 * GWARPS, 0, st>>>(
-      (const float2 *)in, (float2 *)scratch, nrow, ncol, ni, nj, alpha);
-  s = s1b_launch_status();
-  if (s) return s;
-  dim3 grid(nrow, (ncol + 255) / 256);
-  goldstein_gather_kernel<<<grid, 256, 0, st>>>((const float2 *)scratch, (float2 *)out, nrow, ncol, ni, nj);
-  return s1b_launch_status();
+  // every scratch row that the gather reads is written by the kernel before
+  // it, so nothing left by an earlier call needs clearing
+  return launch_goldstein(in, out, nrow, ncol, ni, nj, alpha, scratch, (cudaStream_t)stream);
 }
 
 int frame_goldstein_patch_grid(int nrow, int ncol, int *ni, int *nj) {
@@ -484,12 +566,18 @@ int frame_launch_goldstein(const FrameDev &d, const FrameIO &io, cudaStream_t st
   if (d.n_pairs > 65535 || (d.max_ncol_ml + 255) / 256 > 65535)
     return s1b_fail(S1B_ERR_TOO_LARGE, "frame goldstein: grid too large");
   if (d.max_patches > 0) {
-    dim3 g1((d.max_patches + GWARPS - 1) / GWARPS, d.n_pairs);
-    frame_goldstein_patch_kernel<<<g1, 32 * GWARPS, 0, st>>>(d, io);
+    // CTAs beyond a pair's runs return.  Runs of ni x nj patches: at most 2 nj
+    // (a run of more than ni / 2), or 2 GRUN_JOBS + nj, or ni nj / 8 + nj.
+    const int64_t cols = (d.max_ncol_ml - 1) / GSTEP + 1;
+    const int64_t jobs = std::max<int64_t>(2 * GRUN_JOBS, d.max_patches / GRUN_MAX) + 2 * cols;
+    frame_goldstein_run_kernel<<<dim3((unsigned)std::min<int64_t>(d.max_patches, jobs), d.n_pairs), 32, 0, st>>>(d, io);
     int s = s1b_launch_status();
     if (s) return s;
   }
-  dim3 g2(d.max_nrow_ml, (d.max_ncol_ml + 255) / 256, d.n_pairs);
-  frame_goldstein_gather_kernel<<<g2, 256, 0, st>>>(d, io);
+  const dim3 g2(d.max_nrow_ml, (d.max_ncol_ml - 1) / GGATHER + 1, d.n_pairs);
+  if ((int64_t)d.max_nrow_ml * d.max_ncol_ml * d.n_pairs >= kGatherRows8)
+    frame_goldstein_gather_kernel<GSTEP><<<dim3((d.max_nrow_ml - 1) / GSTEP + 1, g2.y, g2.z), GGATHER, 0, st>>>(d, io);
+  else
+    frame_goldstein_gather_kernel<1><<<g2, GGATHER, 0, st>>>(d, io);
   return s1b_launch_status();
 }

@@ -34,6 +34,24 @@ def test_goldstein_matches_oracle(cuda, shape, alpha):
     assert rel_err(got, want) < 2e-5
 
 
+@pytest.mark.parametrize("shape", [
+    (33, 39),      # clamped last patches one and seven samples after the ones before
+    (40, 64),      # two patch rows: runs of one patch
+    (497, 490),    # runs of two, the last of one
+    (703, 689),    # runs of four
+    (1031, 1048),  # runs of eight, eight output rows per thread, last rows clamped
+])
+def test_goldstein_runs_match_oracle(cuda, shape):
+    """Images either side of the lines between run lengths and between the two
+    gathers (tolerances of the cases above)."""
+    img = _ifg(np.random.default_rng(shape[0]), *shape)
+    got = kernels.goldstein(torch.from_numpy(img).to(cuda), 0.5).cpu().numpy()
+    want = og.goldstein(img, 32, 0.5)
+    m = np.abs(want) > 1e-3 * np.abs(want).max()
+    assert phase_rms(got, want, m) < 1e-3
+    assert rel_err(got, want) < 2e-5
+
+
 def test_goldstein_alpha_zero_and_zeros(cuda):
     rng = np.random.default_rng(2)
     img = _ifg(rng, 48, 64)
