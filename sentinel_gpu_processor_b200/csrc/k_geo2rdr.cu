@@ -409,36 +409,45 @@ __device__ __forceinline__ unsigned geo_warp_setup(const PL &P, const s1b_orbit_
   return cullmask;
 }
 
-// One pixel of a burst's geocoding: ECEF point p of height hgt, tile row r,
-// window column col.  `first` takes the chord slope of this point for the
+// One pixel of a burst's geocoding: ECEF point p of height hgt, tile row rd,
+// hb the seed model's column term.  `first` takes the chord slope of this point for the
 // block (f' changes by < 1e-3 over 32 rows); every point starts from the
 // warp's line model m, within ~1e-6 s of its root.  Returns the geocoded
 // sample, 0 outside the validity window.
 template <typename TSrc, bool kFused, typename PL>
 __device__ __forceinline__ float2 geo_pixel(const PL &P, const GeoConsts &gc,
                                             const ZeroDopplerPatch &zd, const double4 &m, const double p[3],
-                                            double hgt, int r, int col, bool first, double &inv_c1,
+                                            double hgt, double rd, double hb, bool first, double &inv_c1,
                                             const TSrc *__restrict__ burst, const double2 *__restrict__ tops) {
   float2 res = make_float2(0.f, 0.f);
   const ZeroDopplerPoint q = zero_doppler_point(zd, p);
   if (first) inv_c1 = rcp_newton(q.c1);
-  double h = fma(m.w, hgt, fma(m.z, i32_to_f64(r), fma(m.y, i32_to_f64(col), m.x)));
-  const double rng = sqrt_heron(zero_doppler_solve(q, zd.c3, inv_c1, h));
+  double h = fma(m.w, hgt, fma(m.z, rd, hb));
+  const double rng = sqrt_heron(zero_doppler_solve_flat(q, zd.c3, inv_c1, h));
   const double t = zd.t0 + h;
   const double rgoff = (rng - P.rngstart) * gc.inv_dmrg;
   const double azoff = (t - P.tstart) * gc.prf;
-  // validity window, geo2rdr.cu:208-209
-  bool valid = rgoff > P.first_valid_sample && rgoff < P.last_valid_sample - 1 &&
-               azoff >= P.first_valid_line + 5 && azoff < P.last_valid_line - 5;
-  const int intr = (int)rgoff, inta = (int)azoff;
-  // the 2x2 neighbourhood must lie inside the burst even if the validity
-  // limits passed in exceed the raster
-  valid = valid && intr >= 0 && intr + 1 < P.samples && inta >= 0 && inta + 1 < P.lines;
+  // validity window, geo2rdr.cu:208-209, and the 2x2 neighbourhood inside the
+  // burst even if the validity limits passed in exceed the raster; integer
+  // parts as the reference's int() takes them, (-1, 0) to 0, but off the
+  // conversion unit (outside the window they are not used)
+  int intr, inta;
+  double rgi = floor_int(rgoff, intr), azi = floor_int(azoff, inta);
+  bool valid = rgoff > gc.rg_lo && rgoff < gc.rg_hi && azoff >= gc.az_lo && azoff < gc.az_hi;
+  valid = valid && rgoff > -1.0 && intr + 1 < P.samples && azoff > -1.0 && inta + 1 < P.lines;
   if (valid) {
-    const double eta = -P.lines * P.dtaz / 2. + t - P.tstart;
-    const double frd = rgoff - i32_to_f64(intr);
+    if (intr < 0) {
+      intr = 0;
+      rgi = 0.0;
+    }
+    if (inta < 0) {
+      inta = 0;
+      azi = 0.0;
+    }
+    const double eta = gc.eta0 + t - P.tstart;
+    const double frd = rgoff - rgi;
     // bilinear interpolation of the deramped burst (geo2rdr.cu:220-237)
-    const float fr = (float)frd, fa = (float)(azoff - i32_to_f64(inta));
+    const float fr = (float)frd, fa = (float)(azoff - azi);
     const size_t i1 = (size_t)inta * P.samples + intr;
     if constexpr (kFused) {
       // the samples' deramp phases -kt (eta_line - etaref)^2 and the
@@ -446,7 +455,7 @@ __device__ __forceinline__ float2 geo_pixel(const PL &P, const GeoConsts &gc,
       const double2 t0 = __ldg(tops + intr), t1 = __ldg(tops + intr + 1);
       const double ed = eta - fma(frd, t1.y - t0.y, t0.y);
       const double hr = fma(-fma(frd, t1.x - t0.x, t0.x), ed * ed, gc.k4_wvl * rng);
-      const double ea = deramp_eta(P, inta), eb = deramp_eta(P, inta + 1);
+      const double ea = fma(azi, P.ati, gc.ea0), eb = fma(azi + 1.0, P.ati, gc.ea0);
       double d0 = ea - t0.y, d1 = ea - t1.y;
       const double qa0 = t0.x * d0 * d0, qa1 = t1.x * d1 * d1;
       d0 = eb - t0.y;
@@ -511,7 +520,10 @@ __device__ __forceinline__ void geo2rdr_tile(const PL &P, const s1b_orbit_poly_t
   double sinlon, coslon;
   sincos((P.lon0 + col * P.dlon) * kPiD / 180, &sinlon, &coslon);
   const bool colok = col < ncol;
-  const GeoConsts gc = geo_consts(P);
+  __shared__ GeoConsts s_gc;  // read from there per pixel: registers are scarcer
+  if (tx == 0) s_gc = geo_consts(P);
+  __syncthreads();
+  const GeoConsts &gc = s_gc;
   __shared__ ZeroDopplerPatch s_zd[TX / 32];
   __shared__ double4 s_seed[TX / 32];
   const int wid = tx >> 5;
@@ -523,38 +535,45 @@ __device__ __forceinline__ void geo2rdr_tile(const PL &P, const s1b_orbit_poly_t
                                                s_seed[wid]);
   __syncwarp();  // lane 0's patch and seed models are visible to the warp
   const ZeroDopplerPatch &zd = s_zd[wid];
+  const double hb = fma(s_seed[wid].y, i32_to_f64(col), s_seed[wid].x);  // column term of the thread
   double inv_c1 = 0.0;
   int16_t hn = colok && rmax > 0 && !(cullmask & 1u) ? __ldg(dem + (int64_t)row0 * pitch + col) : 0;
   int rlo = INT_MAX, rhi = -1;
-  for (int r = 0; r < rmax; ++r) {
-    if ((r & 31) == 0) {  // a new block of 32 rows (warp-uniform)
-      if ((cullmask >> (r >> 5)) & 1u) {
-        const int rend = min(r + 32, rmax);
-        if (colok)
-          for (; r < rend; ++r) __stcs(out + (size_t)(row0 + r) * ncol + col, make_float2(0.f, 0.f));
-        // the next block's first height (none was loaded ahead)
-        if (colok && r < rmax) hn = __ldg(dem + (int64_t)(row0 + r) * pitch + col);
-        r = rend - 1;
-        continue;
+  for (int rb = 0; rb < rmax; rb += 32) {  // blocks of 32 rows
+    const int rend = min(rb + 32, rmax);
+    if ((cullmask >> (rb >> 5)) & 1u) {  // warp-uniform
+      if (colok)
+        for (int r = rb; r < rend; ++r) __stcs(out + (size_t)(row0 + r) * ncol + col, make_float2(0.f, 0.f));
+      // the next block's first height (none was loaded ahead)
+      if (colok && rend < rmax) hn = __ldg(dem + (int64_t)(row0 + rend) * pitch + col);
+      continue;
+    }
+    if (rb > 0) row_terms(rb);
+    // Two rows per trip, each solve's first two steps straight-line: the second
+    // row's solve overlaps the first one's gathers, whose latency bounds the
+    // loop (3 of 10 stall cycles).  8 dates x bursts of 1500 x 21000: 2380 us
+    // for the stack against 2427 with one row per trip, 2505 with that and the
+    // plan's limits converted and the constants held in registers per pixel;
+    // 2550 at 96 registers and five CTAs per SM.
+#pragma unroll 2
+    for (int r = rb; r < rend; ++r) {
+      const int row = row0 + r;
+      const double sinlat = __shfl_sync(0xffffffffu, r_sin, r & 31);
+      const double coslat = __shfl_sync(0xffffffffu, r_cos, r & 31);
+      const double re = __shfl_sync(0xffffffffu, r_re, r & 31);
+      const double hgt = i32_to_f64(hn);
+      if (colok && r + 1 < rmax) hn = __ldg(dem + (int64_t)(row + 1) * pitch + col);
+      float2 res = make_float2(0.f, 0.f);
+      if (colok) {
+        double p[3];
+        llh_point(sinlat, coslat, re, sinlon, coslon, hgt, p);
+        res = geo_pixel<TSrc, kFused>(P, gc, zd, s_seed[wid], p, hgt, i32_to_f64(r), hb, r == rb, inv_c1, burst, tops);
+        __stcs(out + (size_t)row * ncol + col, res);
       }
-      if (r > 0) row_terms(r);
-    }
-    const int row = row0 + r;
-    const double sinlat = __shfl_sync(0xffffffffu, r_sin, r & 31);
-    const double coslat = __shfl_sync(0xffffffffu, r_cos, r & 31);
-    const double re = __shfl_sync(0xffffffffu, r_re, r & 31);
-    const double hgt = i32_to_f64(hn);
-    if (colok && r + 1 < rmax) hn = __ldg(dem + (int64_t)(row + 1) * pitch + col);
-    float2 res = make_float2(0.f, 0.f);
-    if (colok) {
-      double p[3];
-      llh_point(sinlat, coslat, re, sinlon, coslon, hgt, p);
-      res = geo_pixel<TSrc, kFused>(P, gc, zd, s_seed[wid], p, hgt, r, col, (r & 31) == 0, inv_c1, burst, tops);
-      __stcs(out + (size_t)row * ncol + col, res);
-    }
-    if (res.x != 0.f || res.y != 0.f) {
-      rlo = min(rlo, row);
-      rhi = row + 1;
+      if (res.x != 0.f || res.y != 0.f) {
+        rlo = min(rlo, row);
+        rhi = row + 1;
+      }
     }
   }
   // first / last non-zero output row (geo2rdr.cu:86-128): the warp's extent

@@ -289,6 +289,25 @@ __device__ __forceinline__ double zero_doppler_solve2(const ZeroDopplerPoint &q,
   return fma(-h, fma(fma(fma(0.5 * c3, h, (2.0 / 3.0) * q.c2), h, q.c1), h, 2.0 * q.c0), q.dd);
 }
 
+// zero_doppler_solve with its first two steps straight-line: the same h and
+// squared range, bit by bit, for code that interleaves two solves.
+__device__ __forceinline__ double zero_doppler_solve_flat(const ZeroDopplerPoint &q, double c3, double inv_c1,
+                                                          double &h) {
+  double step = fma(fma(fma(c3, h, q.c2), h, q.c1), h, q.c0) * inv_c1;
+  h -= step;
+  const bool more = !(fabs(step) < 5.0e-9);
+  step = fma(fma(fma(c3, h, q.c2), h, q.c1), h, q.c0) * inv_c1;
+  if (more) h -= step;
+  if (more && !(fabs(step) < 5.0e-9)) {
+    for (int it = 2; it < 51; ++it) {
+      step = fma(fma(fma(c3, h, q.c2), h, q.c1), h, q.c0) * inv_c1;
+      h -= step;
+      if (fabs(step) < 5.0e-9) break;
+    }
+  }
+  return fma(-h, fma(fma(fma(0.5 * c3, h, (2.0 / 3.0) * q.c2), h, q.c1), h, 2.0 * q.c0), q.dd);
+}
+
 // exp(i pi x) of an FP32 phase in half-cycles (|x| < 2^22): the reduction
 // x - 2 rint(x / 2) is exact, then the hardware sine and cosine of the
 // reduced angle (absolute error ~4e-7 on [-pi, pi]).
