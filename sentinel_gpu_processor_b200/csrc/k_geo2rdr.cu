@@ -551,9 +551,9 @@ __device__ __forceinline__ void geo2rdr_tile(const PL &P, const s1b_orbit_poly_t
     if (rb > 0) row_terms(rb);
     // Two rows per trip, each solve's first two steps straight-line: the second
     // row's solve overlaps the first one's gathers, whose latency bounds the
-    // loop (3 of 10 stall cycles).  8 dates x bursts of 1500 x 21000: 2380 us
-    // for the stack against 2427 with one row per trip, 2505 with that and the
-    // plan's limits converted and the constants held in registers per pixel;
+    // loop (3 of 10 stall cycles).  A stack of 4 dates x 2 bursts of 1500 x 21000:
+    // 2380 us against 2427 with one row per trip, 2505 with that and the plan's
+    // limits converted and the constants held in registers per pixel;
     // 2550 at 96 registers and five CTAs per SM.
 #pragma unroll 2
     for (int r = rb; r < rend; ++r) {
