@@ -235,6 +235,15 @@ int s1b_deramp_ci16(const s1b_burst_plan_t *plan, const void *in, void *out, voi
 int s1b_geo2rdr(const s1b_burst_plan_t *plan, const int16_t *dem, int64_t dem_pitch,
                 const void *deramped, void *out, int32_t *rows, void *stream);
 
+/* s1b_deramp and s1b_geo2rdr of both bursts of a pair (reference, secondary),
+ * in two launches; the same bits.  Pointers by burst: slc complex64 [lines *
+ * samples], deramped (written) likewise, dem the window's first pixel (both of
+ * row pitch dem_pitch), out complex64 of the window.  rows: int32[4] device,
+ * the crop rows of the first burst, then of the second. */
+int s1b_geo2rdr_pair(const s1b_burst_plan_t *ref_plan, const s1b_burst_plan_t *sec_plan, const void *const *slc,
+                     void *const *deramped, const int16_t *const *dem, int64_t dem_pitch, void *const *out,
+                     int32_t *rows, void *stream);
+
 /* s1b_deramp and s1b_geo2rdr in one: a burst's raw samples geocoded onto the
  * plan's DEM window, deramped where they are gathered (no deramped copy; the
  * same values within float32 rounding).

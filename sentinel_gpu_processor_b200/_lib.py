@@ -144,6 +144,8 @@ _SIGNATURES = {
     "s1b_deramp": (c_int, [POINTER(BurstPlan), c_void_p, c_void_p, c_void_p]),
     "s1b_deramp_ci16": (c_int, [POINTER(BurstPlan), c_void_p, c_void_p, c_void_p]),
     "s1b_geo2rdr": (c_int, [POINTER(BurstPlan), c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "s1b_geo2rdr_pair": (c_int, [POINTER(BurstPlan), POINTER(BurstPlan), POINTER(c_void_p), POINTER(c_void_p),
+                                 POINTER(c_void_p), c_int64, POINTER(c_void_p), c_void_p, c_void_p]),
     "s1b_geocode_scratch_bytes": (c_size_t, [POINTER(BurstPlan)]),
     "s1b_geocode": (c_int, [POINTER(BurstPlan), c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                             c_size_t, c_void_p]),

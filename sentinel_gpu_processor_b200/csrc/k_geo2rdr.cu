@@ -597,6 +597,64 @@ __global__ __launch_bounds__(G_TX) void geo2rdr_kernel(
   geo2rdr_tile<G_TX, G_RY>(P, P.orbit, dem, pitch, burst, out, rows, nrow, ncol, blockIdx.x, blockIdx.y, cull);
 }
 
+// Both bursts of a pair at once, blockIdx.z = burst: deramp (and the crop rows'
+// start values), then geocoding, with the arithmetic of deramp_kernel and
+// geo2rdr_kernel.  A small burst's launches leave most of the chip idle, each
+// for as long as one tile takes: 331 x 1187 samples, six launches one after
+// the other against two.
+struct PairBurst {
+  const float2 *in;
+  float2 *der;
+  const int16_t *dem;
+  float2 *out;
+  int32_t *rows;
+  int nrow, ncol;
+  bool vec;  // the deramp's wide loads and stores
+};
+
+struct PairArgs {
+  PairBurst b[2];
+  int64_t pitch;
+  bool cull;
+};
+
+__device__ __forceinline__ void deramp_pair_tile(const s1b_burst_plan_t &P, const PairBurst &b) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    b.rows[0] = b.nrow;
+    b.rows[1] = -1;
+  }
+  if ((int)blockIdx.x * 512 >= P.samples || (int)blockIdx.y * DERAMP_ROWS >= P.lines) return;
+  if (b.vec)
+    deramp_tile<true, DERAMP_ROWS>(P, b.in, b.der, blockIdx.x, blockIdx.y);
+  else
+    deramp_tile<false, DERAMP_ROWS>(P, b.in, b.der, blockIdx.x, blockIdx.y);
+}
+
+__global__ __launch_bounds__(256) void deramp_pair_kernel(const __grid_constant__ s1b_burst_plan_t P0,
+                                                          const __grid_constant__ s1b_burst_plan_t P1,
+                                                          const __grid_constant__ PairArgs a) {
+  if (blockIdx.z == 0)
+    deramp_pair_tile(P0, a.b[0]);
+  else
+    deramp_pair_tile(P1, a.b[1]);
+}
+
+__device__ __forceinline__ void geo2rdr_pair_tile(const s1b_burst_plan_t &P, const PairBurst &b, int64_t pitch,
+                                                  bool cull) {
+  if ((int)blockIdx.x * G_TX >= b.ncol || (int)blockIdx.y * G_RY >= b.nrow) return;  // uniform
+  geo2rdr_tile<G_TX, G_RY>(P, P.orbit, b.dem, pitch, b.der, b.out, b.rows, b.nrow, b.ncol, blockIdx.x, blockIdx.y,
+                           cull);
+}
+
+__global__ __launch_bounds__(G_TX) void geo2rdr_pair_kernel(const __grid_constant__ s1b_burst_plan_t P0,
+                                                            const __grid_constant__ s1b_burst_plan_t P1,
+                                                            const __grid_constant__ PairArgs a) {
+  if (blockIdx.z == 0)
+    geo2rdr_pair_tile(P0, a.b[0], a.pitch, a.cull);
+  else
+    geo2rdr_pair_tile(P1, a.b[1], a.pitch, a.cull);
+}
+
 // ------------------------------------------------- geocoding, one launch
 // Deramp and geocoding of one burst without the deramped copy: the raw
 // samples (complex64 or complex int16) are deramped where they are gathered,
@@ -1478,6 +1536,46 @@ extern "C" int s1b_geo2rdr(const s1b_burst_plan_t *plan, const int16_t *dem, int
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr: DEM window too tall");
   geo2rdr_kernel<<<grid, G_TX, 0, st>>>(*plan, dem, dem_pitch, (const float2 *)deramped,
                                          (float2 *)out, rows, nrow, ncol, g_cull_geo != 0);
+  return s1b_launch_status();
+}
+
+extern "C" int s1b_geo2rdr_pair(const s1b_burst_plan_t *ref_plan, const s1b_burst_plan_t *sec_plan,
+                                const void *const *slc, void *const *deramped, const int16_t *const *dem,
+                                int64_t dem_pitch, void *const *out, int32_t *rows, void *stream) {
+  if (!ref_plan || !sec_plan || !slc || !deramped || !dem || !out || !rows)
+    return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_pair: null argument");
+  const s1b_burst_plan_t *plans[2] = {ref_plan, sec_plan};
+  PairArgs a;
+  a.pitch = dem_pitch;
+  a.cull = g_cull_geo != 0;
+  int64_t dx = 0, dy = 0, gx = 0, gy = 0;
+  for (int q = 0; q < 2; ++q) {
+    const s1b_burst_plan_t &p = *plans[q];
+    if (!slc[q] || !deramped[q] || !dem[q] || !out[q])
+      return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_pair: null argument");
+    if (p.samples < 1 || p.lines < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_pair: empty burst");
+    PairBurst &b = a.b[q];
+    b.in = (const float2 *)slc[q];
+    b.der = (float2 *)deramped[q];
+    b.dem = dem[q];
+    b.out = (float2 *)out[q];
+    b.rows = rows + 2 * q;
+    b.nrow = p.win_bottom - p.win_top;
+    b.ncol = p.win_right - p.win_left;
+    b.vec = p.samples % 2 == 0 && (uintptr_t)b.in % 16 == 0 && (uintptr_t)b.der % 16 == 0;
+    if (b.nrow <= 0 || b.ncol <= 0) return s1b_fail(S1B_ERR_EMPTY, "s1b_geo2rdr_pair: empty DEM window");
+    if (dem_pitch < b.ncol) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_pair: dem_pitch < window width");
+    dx = std::max<int64_t>(dx, ((int64_t)p.samples + 511) / 512);
+    dy = std::max<int64_t>(dy, ((int64_t)p.lines + DERAMP_ROWS - 1) / DERAMP_ROWS);
+    gx = std::max<int64_t>(gx, ((int64_t)b.ncol + G_TX - 1) / G_TX);
+    gy = std::max<int64_t>(gy, ((int64_t)b.nrow + G_RY - 1) / G_RY);
+  }
+  if (dy > 65535 || gy > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr_pair: burst or DEM window too tall");
+  cudaStream_t st = (cudaStream_t)stream;
+  deramp_pair_kernel<<<dim3((unsigned)dx, (unsigned)dy, 2), 256, 0, st>>>(*ref_plan, *sec_plan, a);
+  const int s = s1b_launch_status();
+  if (s) return s;
+  geo2rdr_pair_kernel<<<dim3((unsigned)gx, (unsigned)gy, 2), G_TX, 0, st>>>(*ref_plan, *sec_plan, a);
   return s1b_launch_status();
 }
 

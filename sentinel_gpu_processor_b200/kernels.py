@@ -82,6 +82,33 @@ def geo2rdr(plan: _lib.BurstPlan, dem: torch.Tensor, deramped: torch.Tensor, out
     return out, rows
 
 
+def geo2rdr_pair(plans, slcs, dem: torch.Tensor, deramped, outs, rows: torch.Tensor):
+    """:func:`deramp` and :func:`geo2rdr` of both bursts of a pair, in two
+    launches (``s1b_geo2rdr_pair``; the same bits).  ``slcs``, ``deramped`` and
+    ``outs`` are pairs of complex64 tensors, the last two written; ``dem`` the
+    full RSC-grid DEM or the window, if it is both bursts'; ``rows`` int32 [4],
+    written: the crop rows of one burst after the other's."""
+    _need_cuda(dem, rows, *slcs, *deramped, *outs)
+    wins = []
+    for p, slc, der, out in zip(plans, slcs, deramped, outs):
+        for t, name in ((slc, "slc"), (der, "deramped"), (out, "out")):
+            _c64(t, name)
+        if slc.numel() != p.lines * p.samples or der.numel() < slc.numel():
+            raise ValueError("slc size does not match the plan")
+        wins.append(_dem_window(p, dem, "geo2rdr_pair")[0])
+        if out.numel() < wins[-1].numel():
+            raise ValueError("out is smaller than the plan's window")
+    if rows.dtype != torch.int32 or rows.numel() < 4 or not rows.is_contiguous():
+        raise ValueError("rows must be a contiguous int32 [4] tensor")
+
+    def ptrs(ts):
+        return (ctypes.c_void_p * 2)(*[t.data_ptr() for t in ts])
+
+    _lib.check(_call("geo2rdr_pair", _lib.load().s1b_geo2rdr_pair, ctypes.byref(plans[0]), ctypes.byref(plans[1]),
+                     ptrs(slcs), ptrs(deramped), ptrs(wins), wins[0].stride(0), ptrs(outs), _lib.dptr(rows),
+                     _lib.stream_ptr()), "s1b_geo2rdr_pair")
+
+
 def _dem_window(plan: _lib.BurstPlan, dem: torch.Tensor, where: str):
     """The plan's window of ``dem`` (the full RSC-grid DEM or the window itself) and its size."""
     if dem.dtype != torch.int16:
