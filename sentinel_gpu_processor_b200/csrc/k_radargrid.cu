@@ -590,7 +590,7 @@ struct RtSmem {
   float2 win[2][RT_WR][RT_WC];
   float offs[3][2][R_TH][R_TX];
   double mkt[2][RT_WC], eref[2][RT_WC];  // per window stage
-  int4 red[RT_THREADS / 32];
+  int4 red[2][RT_THREADS / 32];  // coordinate ranges per warp, alternating between tiles
   uint64_t bar_off[3], bar_win[2];
 };
 
@@ -696,12 +696,15 @@ __global__ __launch_bounds__(RT_THREADS, 2) void resample_tma_kernel(
     xna = __reduce_max_sync(0xffffffffu, xna);
     mnr = __reduce_min_sync(0xffffffffu, mnr);
     xnr = __reduce_max_sync(0xffffffffu, xnr);
-    if (lane == 0) sm.red[warp] = make_int4(mna, xna, mnr, xnr);
+    // only the barrier below separates one tile's reads from the next tile's
+    // writes (the first two tiles are prepared back to back): hence two sets
+    int4 *red = sm.red[j & 1];
+    if (lane == 0) red[warp] = make_int4(mna, xna, mnr, xnr);
     // generic-proxy writes to the stages that the copies below overwrite are
     // ordered before them by this fence and the barrier
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (__syncthreads_or(!ok_wait)) return false;
-    const int4 all = sm.red[lane & (RT_THREADS / 32 - 1)];
+    const int4 all = red[lane & (RT_THREADS / 32 - 1)];
     mna = __reduce_min_sync(0xffffffffu, all.x);
     xna = __reduce_max_sync(0xffffffffu, all.y);
     mnr = __reduce_min_sync(0xffffffffu, all.z);
