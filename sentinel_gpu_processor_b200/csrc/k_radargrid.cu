@@ -44,7 +44,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 //     range from the same coefficients, instead of two orbit evaluations with
 //     a division each; no row waits for the one above.
 // A pixel off the patch (more than 0.25 s from its centre, or a second step
-// above 1e-6 s) is solved on the orbit polynomials.  The inputs stream through
+// above 1e-6 s) is solved on the orbit polynomials; one without a point (a
+// coordinate that is infinite or no number) yields no number, and no patch is
+// built about it.  The inputs stream through
 // a ring of O_AHEAD rows in shared memory by cp.async (a lane reads back only
 // what it copied itself: no barrier); one row ahead in registers left the FP64
 // pipe waiting for DRAM.  1500 x 21000: 443 -> 288 us (FP64 pipe 49 % busy,
@@ -55,6 +57,11 @@ constexpr int O_TX = 128, O_RY = 64, O_AHEAD = 8;
 // |x| > limit (or x no number), by the high words: off the FP64 pipe.
 __device__ __forceinline__ bool above(double x, double limit) {
   return (__double2hiint(x) & 0x7fffffff) > __double2hiint(limit);
+}
+
+// A geodetic point that a patch can be built about: numbers, and no infinities.
+__device__ __forceinline__ bool usable(double lat, double lon, double h) {
+  return !above(lat, 1.0e6) && !above(lon, 1.0e6) && !above(h, 1.0e9);
 }
 
 // Geodetic point (degrees, metres) to ECEF near a point evaluated in full,
@@ -147,13 +154,33 @@ __global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant_
   const double inv_dmrg = 1.0 / P.dmrg, prf = 1.0 / P.dtaz, cold = col;
   const int rmax = min(O_RY, L - row0);
   ZeroDopplerPatch z;
+  int rc = rmax / 2;  // row of the patch's pixel
   {  // the warp's centre pixel on the orbit polynomials (the same in every lane)
     const int cw = min((int)(blockIdx.x * O_TX + (threadIdx.x & ~31) + 16), S - 1);
-    const size_t i = (size_t)(row0 + rmax / 2) * S + cw;
+    const size_t i = (size_t)(row0 + rc) * S + cw;
+    double la = __ldg(lat + i), lo = __ldg(lon + i), hg = __ldg(hgt + i);
+    if (!usable(la, lo, hg)) {
+      // no point there: the first of the warp's that is one, row by row from
+      // the centre on (none: no patch, every pixel is solved by itself)
+      for (int k = 1; k <= rmax; ++k) {
+        const int r = (rmax / 2 + k) % rmax;
+        const size_t j = (size_t)(row0 + r) * S + col;
+        const double a = __ldg(lat + j), b = __ldg(lon + j), c = __ldg(hgt + j);
+        const unsigned ok = __ballot_sync(0xffffffffu, usable(a, b, c));
+        if (ok) {
+          const int from = __ffs(ok) - 1;
+          la = __shfl_sync(0xffffffffu, a, from);
+          lo = __shfl_sync(0xffffffffu, b, from);
+          hg = __shfl_sync(0xffffffffu, c, from);
+          rc = r;
+          break;
+        }
+      }
+    }
     PointBase base;
     double p[3], up[4], dr[3];
-    base.full(__ldg(lat + i), __ldg(lon + i));
-    base.ecef(base.lat, base.lon, __ldg(hgt + i), p, up);
+    base.full(la, lo);
+    base.ecef(base.lat, base.lon, hg, p, up);
     double t = P.tmid;
     OrbitState st;
 #pragma unroll
@@ -203,7 +230,7 @@ __global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant_
   PointBase base;
   base.full(__ldg(lat + i), __ldg(lon + i));
   double rowd = row0;
-  double hseed = -(rmax / 2) * P.dtaz;  // time of the row from the patch's
+  double hseed = -rc * P.dtaz;  // time of the row from the patch's
   // two rows at a time, so that one's FP64 chain fills the other's gaps
   for (int r0 = 0; r0 < rmax; r0 += 2) {
   double in[2][3];
@@ -231,25 +258,27 @@ __global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant_
       hn -= step;
       on_patch = !above(hn, 0.25) && !above(step, 1.0e-6);
     }
-    double rng;
+    double rng, t = z.t0 + hn;
     if (on_patch) {
       rng = sqrt_heron(fma(-hn, fma(fma(fma(0.5 * z.c3, hn, (2.0 / 3.0) * q.c2), hn, q.c1), hn, 2.0 * q.c0), q.dd));
+    } else if (above(p[0] + p[1] + p[2], 1.0e150)) {
+      t = rng = __longlong_as_double(0x7ff8000000000000LL);  // no point: not a number
     } else {
       OrbitState st;
-      double t = P.tmid, dr[3];
+      double dr[3];
+      t = P.tmid;
       orbit_eval(P.orbit, t, st);
       zero_doppler(P.orbit, p, t, st, dr);
       rng = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-      hn = t - z.t0;
     }
     if (store && r0 + k < rmax) {
       // residuals relative to the pixel index keep float32 at ~1e-5 px
-      __stcs(az_off + i, (float)((z.t0 + hn - P.tstart) * prf - rowd));
+      __stcs(az_off + i, (float)((t - P.tstart) * prf - rowd));
       __stcs(rg_off + i, (float)fma(rng - P.rngstart, inv_dmrg, -cold));
       if (kSens) {
         OrbitState rs, st;
         orbit_eval(R.orbit, R.tstart + rowd * R.dtaz, rs);
-        orbit_eval(P.orbit, z.t0 + hn, st);
+        orbit_eval(P.orbit, t, st);
         const double n[3] = {up[1] * up[3], up[1] * up[2], up[0]};
         const double rr[3] = {p[0] - rs.x[0], p[1] - rs.x[1], p[2] - rs.x[2]};
         const double dr[3] = {p[0] - st.x[0], p[1] - st.x[1], p[2] - st.x[2]};
