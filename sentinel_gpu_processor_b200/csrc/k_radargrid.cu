@@ -32,8 +32,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 }
 
 // -------------------------------------------------------------- offsets
-// Thread = reference column, O_RY rows; one orbit patch per warp (32 columns x
-// O_RY rows, ZeroDopplerPatch) about the zero-Doppler time of its centre pixel.
+// Thread = reference column, ry rows (4 to 64, offsets_rows); one orbit patch
+// per warp (32 columns x ry rows, ZeroDopplerPatch) about the zero-Doppler time
+// of its centre pixel.
 // What bounds it is the FP64 pipe, so a pixel's FP64 operations are what was
 // cut, from about 210 to 85:
 //   * sines and cosines of latitude and longitude and the prime vertical
@@ -49,10 +50,10 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 // built about it.  The inputs stream through
 // a ring of O_AHEAD rows in shared memory by cp.async (a lane reads back only
 // what it copied itself: no barrier); one row ahead in registers left the FP64
-// pipe waiting for DRAM.  1500 x 21000: 443 -> 288 us (FP64 pipe 49 % busy,
-// its latency filled by 16 warps per SM and two rows each; 5 CTAs at 96
-// registers spill: 358; 32 rows per CTA 309, 128 rows 292).
-constexpr int O_TX = 128, O_RY = 64, O_AHEAD = 8;
+// pipe waiting for DRAM.  1500 x 21000: 443 -> 300 us a call (279 back to back;
+// FP64 pipe 49 % busy, its latency filled by 16 warps per SM and two rows each;
+// 5 CTAs at 96 registers spill: 358; 128 rows per CTA 292 against 288 of 64).
+constexpr int O_TX = 128, O_AHEAD = 8, O_CTAS_PER_SM = 4;
 
 // |x| > limit (or x no number), by the high words: off the FP64 pipe.
 __device__ __forceinline__ bool above(double x, double limit) {
@@ -136,11 +137,11 @@ struct RefOrbit {
 };
 
 template <bool kSens>
-__global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant__ s1b_burst_plan_t P,
+__global__ __launch_bounds__(O_TX, O_CTAS_PER_SM) void offsets_kernel(const __grid_constant__ s1b_burst_plan_t P,
                                                        const __grid_constant__ RefOrbit R,
                                                        const double *__restrict__ lat,
                                                        const double *__restrict__ lon,
-                                                       const double *__restrict__ hgt, int L, int S,
+                                                       const double *__restrict__ hgt, int L, int S, int ry,
                                                        float *__restrict__ az_off,
                                                        float *__restrict__ rg_off,
                                                        float *__restrict__ daz_dh,
@@ -150,9 +151,9 @@ __global__ __launch_bounds__(O_TX, 4) void offsets_kernel(const __grid_constant_
   // the last block's spare lanes repeat the last column
   const int col = min((int)(blockIdx.x * O_TX + threadIdx.x), S - 1);
   const bool store = blockIdx.x * O_TX + threadIdx.x < S;
-  const int row0 = blockIdx.y * O_RY;
+  const int row0 = blockIdx.y * ry;
   const double inv_dmrg = 1.0 / P.dmrg, prf = 1.0 / P.dtaz, cold = col;
-  const int rmax = min(O_RY, L - row0);
+  const int rmax = min(ry, L - row0);
   ZeroDopplerPatch z;
   int rc = rmax / 2;  // row of the patch's pixel
   {  // the warp's centre pixel on the orbit polynomials (the same in every lane)
@@ -1412,15 +1413,31 @@ int launch_walk(const void *ref, const void *sec, int lines, int samples, float 
 
 }  // namespace
 
+// Rows per CTA of the offsets: the most, of 4 to 64, that leave enough CTAs.  A
+// CTA starts with its patch, a serial FP64 chain of 3 us, so long CTAs are the
+// cheaper ones (1500 x 21000: 279 us at 64 rows, 298 at 32, 346 at 16) where
+// there are more of them than the SMs hold at once (four each); but each walks
+// its rows in turn, 0.5 us a row, so a small raster takes short ones: 512 x
+// 2048 33 us at 64 rows (128 CTAs), 20 at 32, 16 at 16, 17 at 8; 160 x 640 37
+// us at 64, 7 at 8, 6 at 4.  Two thirds of what the SMs hold is the least that
+// pays (331 x 1187: 13 us at 16 rows, 210 CTAs; 10 at 8, 420; 12 at 4).
+static int offsets_rows(int lines, int samples) {
+  const int64_t cols = (samples - 1) / O_TX + 1, enough = 148 * O_CTAS_PER_SM * 2 / 3;
+  int ry = 64;
+  while (ry > 4 && cols * ((lines - 1) / ry + 1) < enough) ry /= 2;
+  return ry;
+}
+
 extern "C" int s1b_geo2rdr_offsets(const s1b_burst_plan_t *plan, const double *lat, const double *lon,
                                    const double *hgt, int32_t lines, int32_t samples, float *az_off,
                                    float *rg_off, void *stream) {
   if (!plan || !lat || !lon || !hgt || !az_off || !rg_off)
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets: null argument");
   if (lines < 1 || samples < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets: empty grid");
-  dim3 grid((samples + O_TX - 1) / O_TX, (lines + O_RY - 1) / O_RY);
+  const int ry = offsets_rows(lines, samples);
+  dim3 grid((samples + O_TX - 1) / O_TX, (lines + ry - 1) / ry);
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr_offsets: grid too tall");
-  offsets_kernel<false><<<grid, O_TX, 0, (cudaStream_t)stream>>>(*plan, RefOrbit{}, lat, lon, hgt, lines, samples,
+  offsets_kernel<false><<<grid, O_TX, 0, (cudaStream_t)stream>>>(*plan, RefOrbit{}, lat, lon, hgt, lines, samples, ry,
                                                                  az_off, rg_off, nullptr, nullptr);
   return s1b_launch_status();
 }
@@ -1432,13 +1449,14 @@ extern "C" int s1b_geo2rdr_offsets_dh(const s1b_burst_plan_t *plan, const s1b_bu
   if (!plan || !ref_plan || !lat || !lon || !hgt || !az_off || !rg_off || !daz_dh || !drg_dh)
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets_dh: null argument");
   if (lines < 1 || samples < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets_dh: empty grid");
-  dim3 grid((samples + O_TX - 1) / O_TX, (lines + O_RY - 1) / O_RY);
+  const int ry = offsets_rows(lines, samples);
+  dim3 grid((samples + O_TX - 1) / O_TX, (lines + ry - 1) / ry);
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr_offsets_dh: grid too tall");
   RefOrbit ro;
   ro.orbit = ref_plan->orbit;
   ro.tstart = ref_plan->tstart;
   ro.dtaz = ref_plan->dtaz;
-  offsets_kernel<true><<<grid, O_TX, 0, (cudaStream_t)stream>>>(*plan, ro, lat, lon, hgt, lines, samples, az_off,
+  offsets_kernel<true><<<grid, O_TX, 0, (cudaStream_t)stream>>>(*plan, ro, lat, lon, hgt, lines, samples, ry, az_off,
                                                                 rg_off, daz_dh, drg_dh);
   return s1b_launch_status();
 }
