@@ -147,6 +147,7 @@ __global__ __launch_bounds__(O_TX, O_CTAS_PER_SM) void offsets_kernel(const __gr
                                                        float *__restrict__ daz_dh,
                                                        float *__restrict__ drg_dh) {
   __shared__ double s_in[O_AHEAD][3][O_TX];
+  __shared__ double s_snap[O_TX / 32][3];  // kSens: a sixth of the orbit's fourth derivative at each patch's time
   static_assert((O_AHEAD & (O_AHEAD - 1)) == 0, "ring slots are taken modulo a power of two");
   // the last block's spare lanes repeat the last column
   const int col = min((int)(blockIdx.x * O_TX + threadIdx.x), S - 1);
@@ -206,8 +207,10 @@ __global__ __launch_bounds__(O_TX, O_CTAS_PER_SM) void offsets_kernel(const __gr
       const double *c = P.orbit.c[w][k];
       const double snap = fma(fma(fma(840.0 * c[7], tau, 360.0 * c[6]), tau, 120.0 * c[5]), tau, 24.0 * c[4]);
       ds = fma(p[k] - z.x[k], snap, ds);
+      if (kSens && threadIdx.x % 32 == 0) s_snap[threadIdx.x / 32][k] = snap * (1.0 / 6.0);
     }
     z.c3 = fma(ds, 1.0 / 6.0, z.c3);
+    if (kSens) __syncwarp();
   }
   size_t i = (size_t)row0 * S + col;
   size_t inext = i;  // pixel of the next row to copy
@@ -279,7 +282,21 @@ __global__ __launch_bounds__(O_TX, O_CTAS_PER_SM) void offsets_kernel(const __gr
       if (kSens) {
         OrbitState rs, st;
         orbit_eval(R.orbit, R.tstart + rowd * R.dtaz, rs);
-        orbit_eval(P.orbit, t, st);
+        if (on_patch) {
+          // the patch's orbit: 7 multiply-adds a component, the polynomials 21
+          // (1500 x 21000: 636 us back to back, 737 with them).  The velocity to
+          // its h^3 term: between parallel orbits its product with the point's
+          // motion all but cancels (error of daz_dh at most 1.5e-16 lines per
+          // metre, 1.4e-15 without the term, 2.0e-16 with the polynomials)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            st.x[c] = fma(hn, fma(hn, fma(hn, (1.0 / 3.0) * z.jh[c], 0.5 * z.a[c]), z.v[c]), z.x[c]);
+            st.v[c] = fma(hn, fma(hn, fma(hn, s_snap[threadIdx.x / 32][c], z.jh[c]), z.a[c]), z.v[c]);
+            st.a[c] = fma(2.0 * hn, z.jh[c], z.a[c]);
+          }
+        } else {
+          orbit_eval(P.orbit, t, st);
+        }
         const double n[3] = {up[1] * up[3], up[1] * up[2], up[0]};
         const double rr[3] = {p[0] - rs.x[0], p[1] - rs.x[1], p[2] - rs.x[2]};
         const double dr[3] = {p[0] - st.x[0], p[1] - st.x[1], p[2] - st.x[2]};
@@ -1420,9 +1437,14 @@ int launch_walk(const void *ref, const void *sec, int lines, int samples, float 
 // its rows in turn, 0.5 us a row, so a small raster takes short ones: 512 x
 // 2048 33 us at 64 rows (128 CTAs), 20 at 32, 16 at 16, 17 at 8; 160 x 640 37
 // us at 64, 7 at 8, 6 at 4.  Two thirds of what the SMs hold is the least that
-// pays (331 x 1187: 13 us at 16 rows, 210 CTAs; 10 at 8, 420; 12 at 4).
-static int offsets_rows(int lines, int samples) {
-  const int64_t cols = (samples - 1) / O_TX + 1, enough = 148 * O_CTAS_PER_SM * 2 / 3;
+// pays (331 x 1187: 13 us at 16 rows, 210 CTAs; 10 at 8, 420; 12 at 4).  With
+// the sensitivities a row takes twice as long, and what counts is that the CTAs
+// outnumber what the SMs hold by half, so that the last of them do not walk
+// alone (1500 x 4500: 161 us at 64 rows, 864 CTAs; 154 at 32, 1692; 1000 x 3000:
+// 86, 84 and 77 us at 64, 32 and 16 rows).
+static int offsets_rows(int lines, int samples, bool sens) {
+  constexpr int held = 148 * O_CTAS_PER_SM;
+  const int64_t cols = (samples - 1) / O_TX + 1, enough = sens ? held * 3 / 2 : held * 2 / 3;
   int ry = 64;
   while (ry > 4 && cols * ((lines - 1) / ry + 1) < enough) ry /= 2;
   return ry;
@@ -1434,7 +1456,7 @@ extern "C" int s1b_geo2rdr_offsets(const s1b_burst_plan_t *plan, const double *l
   if (!plan || !lat || !lon || !hgt || !az_off || !rg_off)
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets: null argument");
   if (lines < 1 || samples < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets: empty grid");
-  const int ry = offsets_rows(lines, samples);
+  const int ry = offsets_rows(lines, samples, false);
   dim3 grid((samples + O_TX - 1) / O_TX, (lines + ry - 1) / ry);
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr_offsets: grid too tall");
   offsets_kernel<false><<<grid, O_TX, 0, (cudaStream_t)stream>>>(*plan, RefOrbit{}, lat, lon, hgt, lines, samples, ry,
@@ -1449,7 +1471,7 @@ extern "C" int s1b_geo2rdr_offsets_dh(const s1b_burst_plan_t *plan, const s1b_bu
   if (!plan || !ref_plan || !lat || !lon || !hgt || !az_off || !rg_off || !daz_dh || !drg_dh)
     return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets_dh: null argument");
   if (lines < 1 || samples < 1) return s1b_fail(S1B_ERR_INVALID_ARGUMENT, "s1b_geo2rdr_offsets_dh: empty grid");
-  const int ry = offsets_rows(lines, samples);
+  const int ry = offsets_rows(lines, samples, true);
   dim3 grid((samples + O_TX - 1) / O_TX, (lines + ry - 1) / ry);
   if (grid.y > 65535) return s1b_fail(S1B_ERR_TOO_LARGE, "s1b_geo2rdr_offsets_dh: grid too tall");
   RefOrbit ro;
