@@ -487,7 +487,8 @@ size_t s1b_stitch_workspace_bytes(const s1b_stitch_burst_t *bursts, int32_t n, i
  * offset applied to each burst (synchronises the stream when given).  The
  * union box of a subswath is that of its first and last burst, as the
  * reference computes it; parts of middle bursts outside it are dropped.
- * `frame` must not overlap the bursts. */
+ * `frame` may lie over the bursts: it is then formed in memory taken from the
+ * stream's pool (cudaMallocAsync) and copied. */
 int s1b_stitch(const s1b_stitch_burst_t *bursts, int32_t n, const void *data, int32_t out_float, int32_t nrow0,
                int32_t ncol0, void *frame, double *offsets_host, void *workspace, size_t workspace_bytes,
                void *stream);

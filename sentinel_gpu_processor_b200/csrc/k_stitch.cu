@@ -1029,8 +1029,27 @@ extern "C" int s1b_stitch(const s1b_stitch_burst_t *bursts, int32_t n, const voi
     if (e != cudaSuccess) return s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e));
     tab.more = d_b;
   }
-  s = out_float ? launch_stitch<true>(tab, p, data, measured, turns, frame, nrow0, ncol0, st)
-                : launch_stitch<false>(tab, p, data, measured, turns, frame, nrow0, ncol0, st);
+  // The frame is written while bursts are still read: one that lies over any
+  // of them is formed beside them and copied.
+  const size_t es = out_float ? sizeof(float) : sizeof(float2), frame_bytes = (size_t)nrow0 * ncol0 * es;
+  void *formed = frame;
+  for (int i = 0; i < n && formed == frame; ++i) {
+    const s1b_stitch_burst_t &b = bursts[i];
+    const uintptr_t lo = (uintptr_t)data + (uintptr_t)(b.offset * (int64_t)es);
+    const uintptr_t hi = lo + (size_t)(b.right - b.left) * (b.bottom - b.top) * es;
+    if (lo < (uintptr_t)frame + frame_bytes && (uintptr_t)frame < hi) {
+      e = cudaMallocAsync(&formed, frame_bytes, st);
+      if (e != cudaSuccess) return s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e));
+    }
+  }
+  s = out_float ? launch_stitch<true>(tab, p, data, measured, turns, formed, nrow0, ncol0, st)
+                : launch_stitch<false>(tab, p, data, measured, turns, formed, nrow0, ncol0, st);
+  if (formed != frame) {
+    e = s ? cudaSuccess : cudaMemcpyAsync(frame, formed, frame_bytes, cudaMemcpyDeviceToDevice, st);
+    const cudaError_t freed = cudaFreeAsync(formed, st);
+    if (!s && (e != cudaSuccess || freed != cudaSuccess))
+      s = s1b_fail(S1B_ERR_CUDA, cudaGetErrorString(e != cudaSuccess ? e : freed));
+  }
   if (s) return s;
   if (offsets_host) {
     // offsets per burst in the caller's order (the kernel writes them in subswath order)
