@@ -588,7 +588,8 @@ def _e2e_radar(chain, sc, args, world):
     return job_rate(world, k_e2e, chain.burst_pixels, e2e_ms), h2d, d2h
 
 
-KERNELS = ("deramp", "geo2rdr", "crossmul_looks", "goldstein", "geo2rdr_offsets", "resample", "box_coherence")
+KERNELS = ("deramp", "geo2rdr", "geo2rdr_pair", "crossmul_looks", "goldstein", "geo2rdr_offsets", "resample",
+           "box_coherence")
 
 
 def _instrumented(run, steps):
@@ -673,7 +674,8 @@ def _kernel_table(chain, sc, args, times, peak):
         n = len(pls)
         burst = sum(p.lines * p.samples for p in pls) / n
         geo = sum(p.nrow * p.ncol for p in pls) / n
-        bytes_per = {"deramp": 16 * burst, "geo2rdr": GEO_BYTES_PER_GEO_PX * geo + GEO_BYTES_PER_BURST_PX * burst}
+        # the pair's call deramps and geocodes both bursts
+        bytes_per = {"geo2rdr_pair": 2 * (16 * burst + GEO_BYTES_PER_GEO_PX * geo + GEO_BYTES_PER_BURST_PX * burst)}
         if args.config == "frame_pairs":
             res = [r for r in chain.last if r is not None]
             box_px = sum((r.box[2] - r.box[0]) * (r.box[3] - r.box[1]) for r in res) / len(res)
@@ -971,17 +973,16 @@ def run_s1b(args):
                          "geo_px_total": sum(p.nrow * p.ncol for p in chain.plans), "ifg_ml": list(res.ifg.shape)})
         launches = chain.launches_per_step()
     traffic = None
-    if top == "geo2rdr":
-        if frame:  # one launch geocodes every burst
-            if chain.crossmul_fused:
-                ratio = GEO_XMUL_TRAFFIC_RATIO.get(args.samples)
-                traffic = ratio * table["geo2rdr"]["bytes_per_launch"] if ratio and chain.deramp_fused else None
-            else:
-                traffic = (GEO_FUSED_TRAFFIC_RATIO * table["geo2rdr"]["bytes_per_launch"] if chain.deramp_fused
-                           else GEO_DRAM_BYTES_PER_GEO_PX * sum(p.nrow * p.ncol for p in chain.plans))
+    if top == "geo2rdr":  # one launch geocodes every burst of a frame
+        if chain.crossmul_fused:
+            ratio = GEO_XMUL_TRAFFIC_RATIO.get(args.samples)
+            traffic = ratio * table["geo2rdr"]["bytes_per_launch"] if ratio and chain.deramp_fused else None
         else:
-            pls = [p for pl in chain.pairs for p in pl] if args.config == "frame_pairs" else chain.plans
-            traffic = GEO_DRAM_BYTES_PER_GEO_PX * sum(p.nrow * p.ncol for p in pls) / len(pls)
+            traffic = (GEO_FUSED_TRAFFIC_RATIO * table["geo2rdr"]["bytes_per_launch"] if chain.deramp_fused
+                       else GEO_DRAM_BYTES_PER_GEO_PX * sum(p.nrow * p.ncol for p in chain.plans))
+    elif top == "geo2rdr_pair":
+        pls = [p for pl in chain.pairs for p in pl] if args.config == "frame_pairs" else chain.plans
+        traffic = sum(16 * p.lines * p.samples + GEO_DRAM_BYTES_PER_GEO_PX * p.nrow * p.ncol for p in pls) * 2 / len(pls)
     elif top == "resample":
         traffic = RESAMPLE_DRAM_BYTES_PER_PX * chain.burst_pixels
     if frame:
@@ -1005,7 +1006,7 @@ def run_s1b(args):
                      "bytes_per_launch": t["bytes_per_launch"], "launch_ms": t["avg_ms"],
                      "timed": ("CUDA events between the stages of profiled frame runs" if frame
                                else "CUDA events around every launch of the entry point over instrumented eager steps"),
-                     "limiter": GEO_LIMITER if top == "geo2rdr" else "HBM"},
+                     "limiter": GEO_LIMITER if top.startswith("geo2rdr") and top != "geo2rdr_offsets" else "HBM"},
         "kernels": table,
     }
     if frame and top == "geo2rdr" and chain.crossmul_fused and chain.deramp_fused:

@@ -69,19 +69,13 @@ class PairChain:
         self.burst_pixels = L * S
         self._scratch = None
         self._ml_shape = None
-        self.geo_events = None  # list to collect (start, end) CUDA events around geocoding launches
+        self.geo_events = None  # list to collect (start, end) CUDA events around a pair's deramp and geocoding
 
     def geocode(self, ref_slc: torch.Tensor, sec_slc: torch.Tensor, dem: torch.Tensor):
-        if kernels.timer is None and self.geo_events is None:
-            kernels.geo2rdr_pair(self.plans, (ref_slc.reshape(-1), sec_slc.reshape(-1)), dem, self.deramped, self.geo,
-                                 self.rows)
-            return
-        # timed burst by burst
-        for i, (p, slc) in enumerate(zip(self.plans, (ref_slc, sec_slc))):
-            kernels.deramp(p, slc.reshape(-1), out=self.deramped[i])
-            ev = _start_event(self.geo_events)
-            kernels.geo2rdr(p, dem, self.deramped[i], out=self.geo[i], rows=self.rows[2 * i:2 * i + 2])
-            _end_event(self.geo_events, ev)
+        ev = _start_event(self.geo_events)
+        kernels.geo2rdr_pair(self.plans, (ref_slc.reshape(-1), sec_slc.reshape(-1)), dem, self.deramped, self.geo,
+                             self.rows)
+        _end_event(self.geo_events, ev)
 
     def headers(self):
         """Crop rows -> the two ``.gslc`` headers (geo2rdr.cu:641-647), or None if a burst is empty."""
@@ -192,16 +186,10 @@ class FrameChain:
 
     def run_pair(self, k, ref_slc, sec_slc, dem):
         pls = self.pairs[k]
-        if kernels.timer is None and self.geo_events is None:
-            kernels.geo2rdr_pair(pls, (ref_slc.reshape(-1), sec_slc.reshape(-1)), dem, self.deramped,
-                                 [self._geo_view(i, p) for i, p in enumerate(pls)], self.rows[4 * k:4 * k + 4])
-        else:  # timed burst by burst
-            for i, (p, slc) in enumerate(zip(pls, (ref_slc, sec_slc))):
-                kernels.deramp(p, slc.reshape(-1), out=self.deramped[i][:p.lines * p.samples])
-                ev = _start_event(self.geo_events)
-                kernels.geo2rdr(p, dem, self.deramped[i][:p.lines * p.samples], out=self._geo_view(i, p),
-                                rows=self.rows[4 * k + 2 * i:4 * k + 2 * i + 2])
-                _end_event(self.geo_events, ev)
+        ev = _start_event(self.geo_events)
+        kernels.geo2rdr_pair(pls, (ref_slc.reshape(-1), sec_slc.reshape(-1)), dem, self.deramped,
+                             [self._geo_view(i, p) for i, p in enumerate(pls)], self.rows[4 * k:4 * k + 4])
+        _end_event(self.geo_events, ev)
         self.rows_host[4 * k:4 * k + 4].copy_(self.rows[4 * k:4 * k + 4], non_blocking=True)
         torch.cuda.current_stream().synchronize()
         r = self.rows_host[4 * k:4 * k + 4].tolist()
