@@ -6,9 +6,10 @@
 // 0..3) is E_j(v) + t O_j(v) and E_j(v) - t O_j(v), and the derivatives d/df
 // are A_j(v) + t B_j(v) and -A_j(v) + t B_j(v).  E, O, A and B are of degree 4
 // in v and interpolate at the Chebyshev nodes of [0, 1/4] (in extended
-// precision, rounded once): the weights are within 5.5e-8, the derivatives
-// within 8.7e-7, where a table of 1024 bins with linear interpolation is
-// within 4.4e-7 and 9.9e-7 and takes four 128-bit gathers per axis.
+// precision, rounded once).  Evaluated in FP32 as below the weights are within
+// 1.9e-7 and the derivatives within 1.01e-6 (1.01e-7 and 8.9e-7 of it from the
+// rounded coefficients), where a table of 1024 bins with linear interpolation is
+// within 4.9e-7 and 1.1e-6 and takes four 128-bit gathers per axis.
 #ifndef S1B_SINC_CUH
 #define S1B_SINC_CUH
 
