@@ -673,7 +673,11 @@ __global__ __launch_bounds__(G_TX) void geo2rdr_pair_kernel(const __grid_constan
 //   * the deramp of a gathered line and the pixel's reramp as one phase formed
 //     from small differences: with u = eta_line - etaref_c0, w the pixel's
 //     eta - etaref less u, K = kt,
-//       kt_p (u + w)^2 - K0 u^2 = K0 w (2u + w) + frd (K1 - K0) (u + w)^2.
+//       kt_p (u + w)^2 - K0 u^2 = K0 w (2u + w) + (kt_p - K0) (u + w)^2;
+//     kt_p and etaref at the pixel's sample from three columns by a parabola (a
+//     straight line between two is off by kt''/8: 7e-7 rad at the ends of 1530
+//     lines whose FM rate changes by 2 % over 640 samples, which raised the
+//     error of such a burst from 2.0e-7 to 3.0e-7).
 // What bounds it is instruction issue (68 % of slots, FP64 pipe 36 %): 1500 x
 // 21000 complex int16 samples onto 16 M window pixels in 185 us, against 85 us
 // for the deramp and 230 us for the geocoding of the deramped copy; 64-row
@@ -819,15 +823,18 @@ __global__ __launch_bounds__(G_TX, 5) void geocode_kernel(const __grid_constant_
       const float2 s1 = load_ro(src), s2 = load_ro(src + 1);
       const float2 s3 = load_ro(src + P.samples), s4 = load_ro(src + P.samples + 1);
       const double2 k = __ldg(a.tops + intr);
-      const float2 dk = __ldg(a.slopes + intr);
+      const float2 dk = __ldg(a.slopes + intr), dk1 = __ldg(a.slopes + intr + 1);
       const float fr = (float)frd, fa = (float)(azoff - azi);
+      // mean slopes of kt and etaref from the column to the pixel's sample
+      const float hc = fmaf(0.5f, fr, -0.5f);
+      const float kt_f = fmaf(hc, dk1.x - dk.x, dk.x), er_f = fmaf(hc, dk1.y - dk.y, dk.y);
       const double ea = fma(azi, P.ati, gc.ea0);            // deramp_eta of the line
       const double u = ea - k.y;                           // line from its column's reference
-      const double w = fma(-frd, (double)dk.y, gc.eta0 + t - P.tstart - ea);
+      const double w = fma(-frd, (double)er_f, gc.eta0 + t - P.tstart - ea);
       const float e = (float)(u + w), uf = (float)u, k0 = -(float)k.x;
       // the line below: u + ati, w - ati, whose K0 w (2u + w) is less by
       // K0 ati (2u + ati)
-      const double ha = fma(-k.x, w * fma(2.0, u, w), fma(gc.k4_wvl, rng, (double)(fr * dk.x * e * e)));
+      const double ha = fma(-k.x, w * fma(2.0, u, w), fma(gc.k4_wvl, rng, (double)(fr * kt_f * e * e)));
       const double hb2 = fma(k.x, P.ati * fma(2.0, u, P.ati), ha);
       const float2 pa = phasor_quarter(ha), pb = phasor_quarter(hb2);
       // the second column's sample of a line turns by the columns' difference
