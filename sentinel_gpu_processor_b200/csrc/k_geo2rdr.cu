@@ -838,12 +838,13 @@ __global__ __launch_bounds__(G_TX, 5) void geocode_kernel(const __grid_constant_
       const double hb2 = fma(k.x, P.ati * fma(2.0, u, P.ati), ha);
       const float2 pa = phasor_quarter(ha), pb = phasor_quarter(hb2);
       // the second column's sample of a line turns by the columns' difference
-      // K0 de (2u - de) - dk (u - de)^2 (a few 1e-3 half-cycles: FP32)
+      // K0 de (2u - de) - dk (u - de)^2 (a few 1e-3 half-cycles, 0.1 at the ends
+      // of 1530 x 640 samples: FP32)
       const float de = dk.y, ufb = uf + gc.ati_f, ua = uf - de, uc = ufb - de;
       const float ra = fmaf(k0 * de, 2.f * uf - de, -dk.x * ua * ua);
       const float rb = fmaf(k0 * de, 2.f * ufb - de, -dk.x * uc * uc);
-      const float2 ca = cmul(lerp2p(s1, cmul(s2, rotation_pi_f(ra)), fr), pa);
-      const float2 cb = cmul(lerp2p(s3, cmul(s4, rotation_pi_f(rb)), fr), pb);
+      const float2 ca = cmul(lerp2p(s1, cmul(s2, phasor_turn(ra)), fr), pa);
+      const float2 cb = cmul(lerp2p(s3, cmul(s4, phasor_turn(rb)), fr), pb);
       res = lerp2p(ca, cb, fa);
     }
     if (colok) __stcs(dst, res);

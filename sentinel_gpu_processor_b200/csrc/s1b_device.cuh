@@ -80,24 +80,34 @@ __device__ __forceinline__ double floor_int(double x, int &i) {
   return t - 6755399441055744.0;
 }
 
-// Unit phasor exp(i pi h) of an FP64 phase h in half-cycles (|h| < 2^50): the
-// nearest quarter k/2 is taken off in FP64 (k from the low bits of 2 h + 1.5 *
-// 2^52), the rest, |r| <= 1/4, is rounded once (<= 1.5e-8 half-cycles) and sin
-// and cos of pi r are polynomials in r^2 that interpolate at the Chebyshev
-// nodes of [0, 1/16] (computed in extended precision): absolute error below
-// 9e-8, rms 2e-8 each.  Half the instructions of phasor_pi, none of them on
-// the conversion unit but the rounding, and a quarter of its phase rounding.
-__device__ __forceinline__ float2 phasor_quarter(double h) {
-  const double t = fma(h, 2.0, 6755399441055744.0);
-  const int k = __double2loint(t);
-  const float r = (float)fma(-0.5, t - 6755399441055744.0, h);
+// exp(i pi r), |r| <= 1/4: cosine and sine are polynomials in r^2 that
+// interpolate at the Chebyshev nodes of [0, 1/16] (computed in extended
+// precision): absolute error below 9e-8, rms 2e-8 each.
+__device__ __forceinline__ float2 phasor_eighth(float r) {
   const float v = r * r;
   const float s = r * fmaf(v, fmaf(v, fmaf(v, -5.890750992e-01f, 2.549766965e+00f), -5.167707821e+00f), 3.141592644e+00f);
   const float c = fmaf(v, fmaf(v, fmaf(v, fmaf(v, 2.321254140e-01f, -1.335137814e+00f), 4.058710566e+00f),
                                -4.934802197e+00f), 1.f);
-  const float x = k & 1 ? s : c, y = k & 1 ? c : s;
+  return make_float2(c, s);
+}
+
+// Unit phasor exp(i pi h) of an FP64 phase h in half-cycles (|h| < 2^50): the
+// nearest quarter k/2 is taken off in FP64 (k from the low bits of 2 h + 1.5 *
+// 2^52), the rest, |r| <= 1/4, is rounded once (<= 1.5e-8 half-cycles).  Half
+// the instructions of phasor_pi, none of them on the conversion unit but the
+// rounding, and a quarter of its phase rounding.
+__device__ __forceinline__ float2 phasor_quarter(double h) {
+  const double t = fma(h, 2.0, 6755399441055744.0);
+  const int k = __double2loint(t);
+  const float2 p = phasor_eighth((float)fma(-0.5, t - 6755399441055744.0, h));
+  const float x = k & 1 ? p.y : p.x, y = k & 1 ? p.x : p.y;
   return make_float2(__int_as_float(__float_as_int(x) ^ (((k + 1) & 2) << 30)),
                      __int_as_float(__float_as_int(y) ^ ((k & 2) << 30)));
+}
+
+// exp(i pi x) of an FP32 turn in half-cycles, most of them below 1/4.
+__device__ __forceinline__ float2 phasor_turn(float x) {
+  return fabsf(x) <= 0.25f ? phasor_eighth(x) : phasor_quarter((double)x);
 }
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
