@@ -4,12 +4,13 @@
 // (0.5 + 0.5 cos(pi (k - f) / 4)).  They are mirror images, w_k(f) =
 // w_{1-k}(1 - f), so with t = f - 1/2 and v = t^2 the pair k = j + 1, -j (j =
 // 0..3) is E_j(v) + t O_j(v) and E_j(v) - t O_j(v), and the derivatives d/df
-// are A_j(v) + t B_j(v) and -A_j(v) + t B_j(v).  E, O, A and B are of degree 4
-// in v and interpolate at the Chebyshev nodes of [0, 1/4] (in extended
-// precision, rounded once).  Evaluated in FP32 as below the weights are within
-// 1.9e-7 and the derivatives within 1.01e-6 (1.01e-7 and 8.9e-7 of it from the
-// rounded coefficients), where a table of 1024 bins with linear interpolation is
-// within 4.9e-7 and 1.1e-6 and takes four 128-bit gathers per axis.
+// are A_j(v) + t B_j(v) and -A_j(v) + t B_j(v).  E and O are of degree 4 in v, A
+// and B of degree 5, and they interpolate at the Chebyshev nodes of [0, 1/4] (in
+// extended precision, rounded once).  Evaluated in FP32 as below the weights are
+// within 1.9e-7 and the derivatives within 2.0e-7 of them; a table of 1024 bins
+// with linear interpolation is within 4.9e-7 and 1.1e-6 and takes four 128-bit
+// gathers per axis (derivatives of degree 4: 1.01e-6, and 1.1 to 1.8 times the table's
+// error in the mean square).
 #ifndef S1B_SINC_CUH
 #define S1B_SINC_CUH
 
@@ -26,15 +27,17 @@
     {-3.450913596e-03f, -1.461180386e-02f}, {-1.575500278e-04f, 6.822906548e-02f}, {7.028463561e-02f,
     -3.939414541e-02f}, {-6.179815928e-02f, -2.851676288e-04f}, {1.615493810e-02f, 5.410020769e-03f},
 };
-[[maybe_unused]] static __constant__ float2 c_dsinc8[4 * 5] = {
-    {1.316447401e+00f, -9.077257542e-01f}, {-4.157075512e+00f, 1.202532931e-01f}, {2.386238463e+00f,
-    4.646045500e-01f}, {1.950642090e-01f, -3.360972442e-01f}, {-6.631490782e-01f, 8.261869454e-02f},
-    {-1.742653724e-01f, 1.228249694e+00f}, {2.382144502e+00f, -3.849884962e-01f}, {-1.998631491e+00f,
-    -5.647455056e-01f}, {2.699200056e-01f, 4.724721402e-01f}, {3.080874626e-01f, -1.369410292e-01f},
-    {6.172634864e-02f, -3.202104065e-01f}, {-8.844464100e-01f, -1.630983445e-02f}, {9.979949162e-01f,
-    4.694392015e-01f}, {-2.004400475e-01f, -2.568907704e-01f}, {-1.152097402e-01f, 3.743479825e-02f},
-    {-1.461186098e-02f, -3.135329796e-04f}, {2.046962935e-01f, 2.810450376e-01f}, {-1.971883674e-01f,
-    -3.692982459e-01f}, {-3.748554609e-04f, 1.205158743e-01f}, {4.499077020e-02f, 1.688753637e-02f},
+[[maybe_unused]] static __constant__ float2 c_dsinc8[4 * 6] = {
+    {1.316446552e+00f, -9.077258134e-01f}, {-4.156906408e+00f, 1.202647961e-01f}, {2.380842802e+00f,
+    4.642433924e-01f}, {2.553677144e-01f, -3.321071802e-01f}, {-9.383782774e-01f, 6.456524600e-02f},
+    {4.398094776e-01f, 2.865423690e-02f}, {-1.742647798e-01f, 1.228249747e+00f}, {2.382026827e+00f,
+    -3.849987145e-01f}, {-1.994884054e+00f, -5.644276188e-01f}, {2.280949945e-01f, 4.689836808e-01f},
+    {4.987843807e-01f, -1.212380991e-01f}, {-3.044875765e-01f, -2.482252343e-02f}, {6.172607596e-02f,
+    -3.202104851e-01f}, {-8.843923273e-01f, -1.629440105e-02f}, {9.962739779e-01f, 4.689513403e-01f},
+    {-1.812433636e-01f, -2.514744057e-01f}, {-2.026988351e-01f, 1.283687023e-02f}, {1.396497900e-01f,
+    3.915512843e-02f}, {-1.461179888e-02f, -3.134484851e-04f}, {2.046839378e-01f, 2.810283195e-01f},
+    {-1.967943612e-01f, -3.687671139e-01f}, {-4.776554293e-03f, 1.145979051e-01f}, {6.507418728e-02f,
+    4.383598285e-02f}, {-3.208509976e-02f, -4.298684190e-02f},
 };
 
 // The 8 weights at the fraction f in [0, 1).
@@ -58,10 +61,10 @@ __device__ __forceinline__ void sinc8_slopes(float fa, float fr, float da[8], fl
   const float2 va2 = make_float2(va, va), vr2 = make_float2(vr, vr);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    float2 a = c_dsinc8[j * 5 + 4], r = a;
+    float2 a = c_dsinc8[j * 6 + 5], r = a;
 #pragma unroll
-    for (int k = 3; k >= 0; --k) {
-      const float2 ck = c_dsinc8[j * 5 + k];
+    for (int k = 4; k >= 0; --k) {
+      const float2 ck = c_dsinc8[j * 6 + k];
       a = __ffma2_rn(a, va2, ck);
       r = __ffma2_rn(r, vr2, ck);
     }

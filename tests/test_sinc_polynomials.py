@@ -1,6 +1,7 @@
 """The polynomials of the 8-tap windowed-sinc weights and their derivatives
 (csrc/s1b_sinc.cuh), evaluated in float32 as the kernels do, against the
-definition in float64: within the bounds that the header states."""
+definition in float64: within the bounds that the header states, and in the
+mean square no farther than a table of 1024 bins with linear interpolation."""
 import os
 import re
 
@@ -12,8 +13,8 @@ SRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), os.pardir, "senti
 
 
 def _table(text, name):
-    body = re.search(name + r"\[4 \* 5\] = \{(.*?)\};", text, re.S).group(1)
-    return np.array([float(x) for x in re.findall(r"-?\d\.\d+e[+-]\d+", body)], dtype=np.float32).reshape(4, 5, 2)
+    n, body = re.search(name + r"\[4 \* (\d)\] = \{(.*?)\};", text, re.S).groups()
+    return np.array([float(x) for x in re.findall(r"-?\d\.\d+e[+-]\d+", body)], dtype=np.float32).reshape(4, int(n), 2)
 
 
 def _definition(f):
@@ -39,8 +40,8 @@ def _evaluate(table, f, even):
     v = t * t
     out = [None] * 8
     for j in range(4):
-        p, q = (np.full_like(f, table[j, 4, i]) for i in (0, 1))
-        for k in (3, 2, 1, 0):
+        p, q = (np.full_like(f, table[j, -1, i]) for i in (0, 1))
+        for k in range(table.shape[1] - 2, -1, -1):
             p, q = _fma(p, v, table[j, k, 0]), _fma(q, v, table[j, k, 1])
         out[4 + j] = _fma(t, q, p)
         out[3 - j] = _fma(-t, q, p) if even else _fma(t, q, -p)
@@ -61,3 +62,15 @@ def test_within_the_stated_bound(text, name, which):
     f = np.append(np.arange(1 << 17) / (1 << 17), 1 - 2.0 ** -24).astype(np.float32)
     got = _evaluate(_table(text, name), f, even=which == 0)
     assert np.abs(got - _definition(f.astype(np.float64))[which]).max() <= bound
+
+
+@pytest.mark.parametrize("name,which", [("c_sinc8", 0), ("c_dsinc8", 1)])
+def test_no_farther_than_a_table(text, name, which):
+    f = ((np.arange(1 << 16) + 0.5) / (1 << 16)).astype(np.float32)
+    want = _definition(f.astype(np.float64))[which]
+    bins = _definition(np.arange(1025) / 1024)[which].astype(np.float32)
+    pos = f * np.float32(1024)
+    b = pos.astype(np.int64)
+    lerp = _fma(pos - b.astype(np.float32), bins[:, b + 1] - bins[:, b], bins[:, b])
+    rms = lambda e: np.sqrt((e ** 2).mean(1))  # noqa: E731
+    assert np.all(rms(_evaluate(_table(text, name), f, even=which == 0) - want) <= rms(lerp - want))
