@@ -227,7 +227,7 @@ __device__ __noinline__ void interp_direct(const s1b_burst_plan_t &P, const floa
 // about half of all 900.  So that three CTAs fit an SM (80 registers, 62 KB)
 // the pixel loop stays rolled and carries a pixel's coordinates and results
 // through shared memory, where the products take the window's place: two
-// bursts of 1468 x 20968 pixels in 2.41 ms (61 % of issue slots; with two CTAs
+// bursts of 1468 x 20968 pixels in 2.42 ms (61 % of issue slots; with two CTAs
 // at 128 registers 2.78).  Before, with the weights and their derivatives in
 // tables whose bins lay 32 bytes apart, coordinates in local memory and one
 // thread per window summing its four products, 4.46 ms at 39 %, half of the
